@@ -273,7 +273,8 @@ long long wb_kernel_launches(wb_handle* h);
  * complex products from the tensor cores (split TF32) to FP32 SIMT, which changes their rounding
  * within FP32 accuracy. No counterpart in the reference (its backends leave launch shapes to
  * LAPACK and torch). */
-#define WB_TUNE_QR_THREADS 0     /* threads of a QR-sweep CTA (64..1024, multiple of 32) */
+#define WB_TUNE_QR_THREADS 0     /* threads of a QR-sweep CTA (64..1024, multiple of 32; held to 128..512 in
+                                    FP32 and 128..256 in the other forms) */
 #define WB_TUNE_HRD_THREADS 1    /* threads of a Hessenberg-reduction CTA (64..1024, multiple of 32) */
 #define WB_TUNE_LU_THREADS 2     /* reserved: threads of an LU / triangular-solve CTA */
 #define WB_TUNE_TENSOR_CORES 3   /* 1: FP32 complex products on the SIMT kernel instead of tcgen05 */
