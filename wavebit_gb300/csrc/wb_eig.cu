@@ -142,8 +142,10 @@ __device__ __forceinline__ Cx<R> column_dot(const Cx<R>* v, const Cx<R>* c, int 
 
 template <class R>
 __global__ void __launch_bounds__(1024) gehrd_kernel(Cx<R>* __restrict__ Aall, int n, int lda,
-                                                     long long a_bs, Cx<R>* __restrict__ tau_all) {
+                                                     long long a_bs, Cx<R>* __restrict__ tau_all,
+                                                     const int* __restrict__ live) {
   using C_ = Cx<R>;
+  if (live && (int)blockIdx.x >= *live) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   C_* sv = reinterpret_cast<C_*>(smraw);          // v (n), then y = A v (n)
   __shared__ R red[32];
@@ -463,8 +465,10 @@ __global__ void clear_below_subdiag_kernel(Cx<R>* __restrict__ Aall, int n, int 
 template <class R>
 __global__ void __launch_bounds__(1024) unghr_kernel(Cx<R>* __restrict__ Aall, int n, int lda,
                                                             long long a_bs, const Cx<R>* __restrict__ tau_all,
-                                                            Cx<R>* __restrict__ Zall, int ldz, long long z_bs) {
+                                                            Cx<R>* __restrict__ Zall, int ldz, long long z_bs,
+                                                            const int* __restrict__ live) {
   using C_ = Cx<R>;
+  if (live && (int)blockIdx.x >= *live) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   C_* sv = reinterpret_cast<C_*>(smraw);
   C_* A = Aall + blockIdx.x * a_bs;
@@ -515,8 +519,9 @@ template <class R>
 __global__ void __launch_bounds__(256) hseqr_small_kernel(Cx<R>* __restrict__ Hall, int n, int ldh,
                                                             long long h_bs, Cx<R>* __restrict__ Zall, int ldz,
                                                             long long z_bs, Cx<R>* __restrict__ w_all,
-                                                            int32_t* __restrict__ status, int st_div, int itmax) {
+                                                            int32_t* __restrict__ status, int st_div, int itmax, const int* __restrict__ live) {
   using C_ = Cx<R>;
+  if (live && (int)blockIdx.x >= *live) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   C_* sphase = reinterpret_cast<C_*>(smraw);
   __shared__ int ired[32];
@@ -745,13 +750,14 @@ __global__ void __launch_bounds__(256) hseqr_small_kernel(Cx<R>* __restrict__ Ha
 template <class R>
 __global__ void __launch_bounds__(256) trevc_kernel(const Cx<R>* __restrict__ Tall, int n, int ldt,
                                                     long long t_bs, Cx<R>* __restrict__ Xall, int ldx,
-                                                    long long x_bs, int batch) {
+                                                    long long x_bs, int batch, const int* __restrict__ live) {
   using C_ = Cx<R>;
   const int warps_per_block = blockDim.x >> 5;
   long long gw = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (gw >= (long long)batch * n) return;
   const int b = (int)(gw / n), k = (int)(gw % n);
+  if (live && b >= *live) return;
   const C_* T = Tall + b * t_bs;
   C_* x = Xall + b * x_bs + (long long)k * ldx;
   const R ulp = RealT<R>::eps();
@@ -796,13 +802,15 @@ __global__ void __launch_bounds__(256) trevc_kernel(const Cx<R>* __restrict__ Ta
 
 // ------------------------------------------------------------- 5. column normalisation
 template <class R>
-__global__ void normalize_columns_kernel(Cx<R>* __restrict__ Wall, int n, int ldw, long long w_bs, int batch) {
+__global__ void normalize_columns_kernel(Cx<R>* __restrict__ Wall, int n, int ldw, long long w_bs, int batch,
+                                         const int* __restrict__ live) {
   using C_ = Cx<R>;
   const int warps_per_block = blockDim.x >> 5;
   long long gw = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (gw >= (long long)batch * n) return;
   const int b = (int)(gw / n), k = (int)(gw % n);
+  if (live && b >= *live) return;
   C_* c = Wall + b * w_bs + (long long)k * ldw;
   R s = R(0.0);
   for (int r = lane; r < n; r += 32) s = s + cxabs2(c[r]);
@@ -892,7 +900,8 @@ int hrd_threads(int batch, int n) {
 
 template <class R>
 void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a_bs, Cx<R>* Z, int ldz,
-                long long z_bs, Cx<R>* w, Cx<R>* tau, int32_t* status, int st_div, Cx<R>* ws, long long ws_bs) {
+                long long z_bs, Cx<R>* w, Cx<R>* tau, int32_t* status, int st_div, Cx<R>* ws, long long ws_bs,
+                const int* live) {
   if (batch <= 0 || n <= 0) return;
   size_t sm = 2 * (size_t)n * sizeof(Cx<R>);
   cudaFuncSetAttribute(gehrd_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -926,7 +935,7 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
       gemm<R>(s, batch, rows, m, bb, mone, V + (k + 1), 1, n, z_bs, Xm, 1, BB, z_bs, one, Ac + (k + 1), 1, lda, a_bs);
     }
   } else {
-    gehrd_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau); note_launch();
+    gehrd_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, live); note_launch();
   }
   // Q in panels when the caller lends scratch (5 n kHrdPanel + kHrdPanel^2 elements a matrix)
   if (blocked && ws && ws_bs >= 5LL * n * kHrdPanel + kHrdPanel * kHrdPanel) {
@@ -952,7 +961,7 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
     const unsigned gx = (unsigned)min((long long)sm_count(), ((long long)n * n + 255) / 256);
     clear_below_subdiag_kernel<R><<<dim3(gx, batch), 256, 0, s>>>(A, n, lda, a_bs); note_launch();
   } else {
-    unghr_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, Z, ldz, z_bs); note_launch();
+    unghr_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, Z, ldz, z_bs, live); note_launch();
   }
   int itmax = 30 * (n > 10 ? n : 10);
   const QrShape shape = qr_shape<R>(batch, n);
@@ -982,7 +991,7 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
   if constexpr (std::is_same<R, double>::value) {
     if (n <= kQrSmall) {
       hseqr_small_kernel<R><<<batch, 128, (size_t)n * sizeof(Cx<R>), s>>>(A, n, lda, a_bs, Z, ldz, z_bs, w, status,
-                                                                         st_div < 1 ? 1 : st_div, itmax);
+                                                                         st_div < 1 ? 1 : st_div, itmax, live);
       launched = true;
     }
   }
@@ -994,17 +1003,17 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
 
 template <class R>
 void trevc(cudaStream_t s, int batch, int n, const Cx<R>* T, int ldt, long long t_bs, Cx<R>* X, int ldx,
-           long long x_bs) {
+           long long x_bs, const int* live) {
   long long warps = (long long)batch * n;
   if (warps <= 0) return;
-  trevc_kernel<R><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(T, n, ldt, t_bs, X, ldx, x_bs, batch); note_launch();
+  trevc_kernel<R><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(T, n, ldt, t_bs, X, ldx, x_bs, batch, live); note_launch();
 }
 
 template <class R>
-void normalize_columns(cudaStream_t s, int batch, int n, Cx<R>* W, int ldw, long long w_bs) {
+void normalize_columns(cudaStream_t s, int batch, int n, Cx<R>* W, int ldw, long long w_bs, const int* live) {
   long long warps = (long long)batch * n;
   if (warps <= 0) return;
-  normalize_columns_kernel<R><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(W, n, ldw, w_bs, batch); note_launch();
+  normalize_columns_kernel<R><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(W, n, ldw, w_bs, batch, live); note_launch();
 }
 
 // double2 wrappers of the plain FP64 path
@@ -1023,9 +1032,10 @@ void znormalize_columns(cudaStream_t s, int batch, int n, cplx* W, int ldw, long
 
 #define WB_EIG_INST(R)                                                                                   \
   template void geev_schur<R>(cudaStream_t, int, int, Cx<R>*, int, long long, Cx<R>*, int, long long,     \
-                              Cx<R>*, Cx<R>*, int32_t*, int, Cx<R>*, long long);                          \
-  template void trevc<R>(cudaStream_t, int, int, const Cx<R>*, int, long long, Cx<R>*, int, long long);  \
-  template void normalize_columns<R>(cudaStream_t, int, int, Cx<R>*, int, long long);
+                              Cx<R>*, Cx<R>*, int32_t*, int, Cx<R>*, long long, const int*);              \
+  template void trevc<R>(cudaStream_t, int, int, const Cx<R>*, int, long long, Cx<R>*, int, long long,   \
+                         const int*);                                                                    \
+  template void normalize_columns<R>(cudaStream_t, int, int, Cx<R>*, int, long long, const int*);
 WB_EIG_INST(double)
 WB_EIG_INST(float)
 WB_EIG_INST(df64)

@@ -781,13 +781,24 @@ __global__ void vmodes_epilogue_kernel(long long total, int N, int n, const int*
   V[idx] = cdiv(v, q[p * n + j]);
 }
 
-// every slot a diagonal 32 x 32 block with distinct entries, so unused slots converge at once
-__global__ void group_init_kernel(int cap, cplx* __restrict__ A, int* __restrict__ count) {
-  long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx == 0) { count[0] = 0; count[1] = 0; }
-  if (idx >= (long long)cap * kGroupMax * kGroupMax) return;
-  const int rem = (int)(idx % (kGroupMax * kGroupMax)), a = rem % kGroupMax, b = rem / kGroupMax;
-  A[idx] = (a == b) ? cmk(1.0 + a, 0.0) : cmk(0.0, 0.0);
+// The eigenvectors Z X of the used slots' blocks, into A (one CTA a slot)
+__global__ void __launch_bounds__(256) group_product_kernel(const cplx* __restrict__ Zall, const cplx* __restrict__ Xall,
+                                                            cplx* __restrict__ Aall, const int* __restrict__ live) {
+  __shared__ cplx z[kGroupMax][kGroupMax + 1], x[kGroupMax][kGroupMax + 1];
+  if ((int)blockIdx.x >= *live) return;
+  const long long o = (long long)blockIdx.x * kGroupMax * kGroupMax;
+  for (int e = threadIdx.x; e < kGroupMax * kGroupMax; e += blockDim.x) {
+    z[e / kGroupMax][e % kGroupMax] = Zall[o + e];            // [column][row]
+    x[e / kGroupMax][e % kGroupMax] = Xall[o + e];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < kGroupMax * kGroupMax; e += blockDim.x) {
+    const int r = e % kGroupMax, c = e / kGroupMax;
+    cplx acc = cmk(0.0, 0.0);
+#pragma unroll 8
+    for (int k = 0; k < kGroupMax; ++k) acc = cfma(z[k][r], x[c][k], acc);
+    Aall[o + e] = acc;
+  }
 }
 
 // One CTA per pair: d, the groups (lock-free union-find over the strong couplings, links always
@@ -865,6 +876,7 @@ __global__ void __launch_bounds__(256) group_kernel(int n, const Cx<float>* __re
       slot[r] = sl; gb.pair[sl] = p; gb.size[sl] = cnt[r];
     } else {
       s_fail = 1;
+      if (sl < gb.cap) gb.offmax[sl] = 0.0;      // too large a group: its slot is left unused
     }
   }
   __syncthreads();
@@ -1094,8 +1106,7 @@ void stage_b_newton(cudaStream_t s, int P, int N, const cplx* conv, const int* p
                                                     (const cplx*)Ym, Wd, nb.lam, nb.F4);
     note_launch();
     getrs<float>(s, P, n, nb.F1, n, n2, nb.piv, n, nb.F4, n, n, n2, 0);            // G = W32^-1 R
-    group_init_kernel<<<nblk((long long)gb.cap * kGroupMax * kGroupMax, 256), 256, 0, s>>>(gb.cap, gb.A, gb.count);
-    note_launch();
+    cudaMemsetAsync(gb.count, 0, 2 * sizeof(int), s);
     group_kernel<<<P, 256, gsm, s>>>(n, nb.F4, nb.lam, nb.F3, gb, st, st_div); note_launch();
     gemm<float>(s, P, n, n, n, one, nb.F2, 1, n, n2, nb.F3, 1, n, n2, zero, nb.F4, 1, n, n2);   // W E
     accumulate_kernel<float, double><<<nblk(tot, 256), 256, 0, s>>>(tot, nb.F4, (Cx<double>*)Wd); note_launch();
@@ -1104,12 +1115,13 @@ void stage_b_newton(cudaStream_t s, int P, int N, const cplx* conv, const int* p
     Cx<double>* Zs = (Cx<double>*)gb.Z;
     Cx<double>* Xs = (Cx<double>*)gb.X;
     const long long b2 = (long long)kGroupMax * kGroupMax;
+    // (of the used slots: the pool is sized for the worst case and nearly empty as a rule; worked on
+    // whole it took 8 of an orders-(5,5) request's 78 ms)
     geev_schur<double>(s, gb.cap, kGroupMax, A, kGroupMax, b2, Zs, kGroupMax, b2, (Cx<double>*)gb.w,
-                       (Cx<double>*)gb.tau, nullptr, 1);
-    trevc<double>(s, gb.cap, kGroupMax, A, kGroupMax, b2, Xs, kGroupMax, b2);
-    gemm<double>(s, gb.cap, kGroupMax, kGroupMax, kGroupMax, one, Zs, 1, kGroupMax, b2, Xs, 1, kGroupMax, b2, zero,
-                 A, 1, kGroupMax, b2);
-    normalize_columns<double>(s, gb.cap, kGroupMax, A, kGroupMax, b2);
+                       (Cx<double>*)gb.tau, nullptr, 1, nullptr, 0, gb.count);
+    trevc<double>(s, gb.cap, kGroupMax, A, kGroupMax, b2, Xs, kGroupMax, b2, gb.count);
+    group_product_kernel<<<gb.cap, 256, 0, s>>>(gb.Z, gb.X, gb.A, gb.count); note_launch();
+    normalize_columns<double>(s, gb.cap, kGroupMax, A, kGroupMax, b2, gb.count);
     group_apply_kernel<<<gb.cap, 256, 0, s>>>(n, n2, gb, Wd, nb.lam, st, st_div); note_launch();
     group2_apply_kernel<<<nblk(32LL * gb.cap2, 256), 256, 0, s>>>(n, n2, gb, Wd, nb.lam); note_launch();
     normalize_columns<double>(s, P, n, (Cx<double>*)Wd, n, n2);
