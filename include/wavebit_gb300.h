@@ -269,22 +269,22 @@ long long wb_kernel_launches(wb_handle* h);
 
 /* Launch-shape tunables, process-wide: 0 restores the library's own choice. The autotuner
  * (wavebit_gb300/autotune.py) times candidates per (orders, layers, batch) bucket and sets them
- * before each batch. Thread counts never change a result; WB_TUNE_TENSOR_CORES = 1 moves the FP32
- * complex products from the tensor cores (split TF32) to FP32 SIMT, which changes their rounding
- * within FP32 accuracy. No counterpart in the reference (its backends leave launch shapes to
+ * before each batch. Thread counts never change a result; WB_TUNE_TENSOR_CORES = 1 moves the
+ * complex products from the tensor cores (FP32: split TF32; FP64: exact slices) to FP32 and FP64 SIMT,
+ * which changes their rounding within FP32 (FP64) accuracy. No counterpart in the reference (its backends leave launch shapes to
  * LAPACK and torch). */
 #define WB_TUNE_QR_THREADS 0     /* threads of a QR-sweep CTA (64..1024, multiple of 32; held to 128..512 in
                                     FP32 and 128..256 in the other forms) */
 #define WB_TUNE_HRD_THREADS 1    /* threads of a Hessenberg-reduction CTA (64..1024, multiple of 32) */
 #define WB_TUNE_LU_THREADS 2     /* reserved: threads of an LU / triangular-solve CTA */
-#define WB_TUNE_TENSOR_CORES 3   /* 1: FP32 complex products on the SIMT kernel instead of tcgen05 */
+#define WB_TUNE_TENSOR_CORES 3   /* 1: complex products on the SIMT kernels instead of tcgen05 */
 #define WB_TUNE_HRD_BLOCKED 4    /* 1: the FP32 Hessenberg reduction one column at a time instead of in panels */
 #define WB_TUNE_COUNT 8
 int wb_set_tuning(int key, int value);
 /* The current value of a tunable (0 = the library's own choice), or -1 for an unknown key. */
 int wb_get_tuning(int key);
 
-/* CTAs of the tensor-core complex product (tcgen05, 3xTF32) whose bounded wait on their own
+/* CTAs of the tensor-core complex products (tcgen05, FP32 and FP64) whose bounded wait on their own
  * MMAs ran out since the library was loaded (they skip their output and raise this count); 0 in
  * a healthy run, -1 if the counter cannot be read. No counterpart in the reference. */
 long long wb_tensor_core_errors(void);

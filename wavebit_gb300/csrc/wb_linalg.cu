@@ -156,6 +156,11 @@ void gemm(cudaStream_t s, int batch, int m, int n, int k, double2 alpha,
                  b_bs, beta, (Cx<float>*)C, c_rs, c_cs, c_bs))
       return;
   }
+  if constexpr (std::is_same<R, double>::value) {   // FP64: exact slices on the tensor cores
+    if (oz_zgemm(s, batch, m, n, k, alpha, (const cplx*)A, a_rs, a_cs, a_bs, nullptr, false, (const cplx*)B, b_rs, b_cs,
+                 b_bs, false, beta, (cplx*)C, c_rs, c_cs, c_bs))
+      return;
+  }
   if (n <= 8 && k > 0 && a_rs == 1 && b_rs == 1 && c_rs == 1) {
     dim3 g((m + NW_ROWS - 1) / NW_ROWS, batch);
     if (n <= 3)
@@ -180,6 +185,11 @@ void gemm_idx(cudaStream_t s, int batch, int m, int n, int k, double2 alpha,
               const Cx<R>* B, long long b_rs, long long b_cs, long long b_bs,
               double2 beta, Cx<R>* C, long long c_rs, long long c_cs, long long c_bs) {
   if (batch <= 0 || m <= 0 || n <= 0) return;
+  if constexpr (std::is_same<R, double>::value) {
+    if (oz_zgemm(s, batch, m, n, k, alpha, (const cplx*)A, a_rs, a_cs, a_bs, a_idx, false, (const cplx*)B, b_rs, b_cs,
+                 b_bs, false, beta, (cplx*)C, c_rs, c_cs, c_bs))
+      return;
+  }
   dim3 grid((m + GT - 1) / GT, (n + GT - 1) / GT, batch);
   gemm_kernel<R><<<grid, 256, 0, s>>>(m, n, k, alpha, A, a_rs, a_cs, a_bs, B, b_rs, b_cs, b_bs, beta, C, c_rs,
                                       c_cs, c_bs, a_idx); note_launch();
@@ -684,6 +694,13 @@ void getrf(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a_bs, 
     }
     const int m = n - k0 - kb;
     if (m > 0) {
+      const int c0 = k0 + kb;
+      if constexpr (std::is_same<R, double>::value) {   // A22 -= L21 U12
+        if (oz_zgemm(s, batch, m, m, kb, make_double2(-1.0, 0.0), (const cplx*)A + c0 + (long long)k0 * lda, 1, lda,
+                     a_bs, nullptr, false, (const cplx*)A + k0 + (long long)c0 * lda, 1, lda, a_bs, false,
+                     make_double2(1.0, 0.0), (cplx*)A + c0 + (long long)c0 * lda, 1, lda, a_bs))
+          continue;
+      }
       dim3 g3((m + GT - 1) / GT, (m + GT - 1) / GT, batch);
       lu_update_kernel<R><<<g3, 256, 0, s>>>(A, n, lda, a_bs, k0, kb);
       note_launch();
@@ -1136,6 +1153,9 @@ void zgemm_conj(cudaStream_t s, int batch, int m, int n, int k, cplx alpha, cons
     zgemm(s, batch, m, n, k, alpha, A, a_rs, a_cs, a_bs, B, b_rs, b_cs, b_bs, beta, C, c_rs, c_cs, c_bs);
     return;
   }
+  if (oz_zgemm(s, batch, m, n, k, alpha, A, a_rs, a_cs, a_bs, nullptr, conj_a, B, b_rs, b_cs, b_bs, conj_b, beta, C,
+               c_rs, c_cs, c_bs))
+    return;
   using D = Cx<double>;
   const D* a = (const D*)A;
   const D* b = (const D*)B;
