@@ -11,6 +11,7 @@
 #include "wb_common.cuh"
 #include "wb_num.cuh"
 #include "wb_kernels.h"
+#include "wb_tri.cuh"
 
 namespace wb {
 
@@ -464,156 +465,14 @@ __global__ void __launch_bounds__(LU_THREADS) getrf_kernel(
 // ------------------------------------------------ LU across the GPU for small batches
 // When a batch holds fewer matrices than the GPU has room for (the cascade factors one layer of
 // every solve at a time), one CTA per matrix leaves most SMs idle. The blocked right-looking LU
-// then runs as three launches per panel of LU_PB columns:
-//   lu_panel_kernel      one CTA per matrix: partial pivoting down the panel, swaps inside it
-//   lu_swap_trsm_kernel  one thread per column outside the panel: the panel's row swaps, then
+// then runs as three launches per panel of LU_PB columns (wb_tri.cuh):
+//   lu_panel_kernel      a cluster of CTAs per matrix: partial pivoting down the panel
+//   lu_swap_trsm_kernel  8 threads per column outside the panel: the panel's row swaps, then
 //                        U12 = L11^-1 A12 for the trailing columns
-//   lu_update_kernel     A22 -= L21 U12 in 64 x 64 tiles over every SM
+//   the update           A22 -= L21 U12: in FP64 the tensor-core product, else lu_update_kernel's 64 x 64
+//                        tiles, over every SM
 // The pivots are the single-CTA kernel's (largest |re| + |im|, first index on ties).
-constexpr int LU_PB = 32;            // panel width
-constexpr int LU_PANEL_THREADS = 1024;
-
-namespace {
-__device__ __forceinline__ double lu_shfl_down(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
-__device__ __forceinline__ float lu_shfl_down(float v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
-__device__ __forceinline__ df64 lu_shfl_down(df64 v, int o) {
-  return df64(__shfl_down_sync(0xffffffffu, v.hi, o), __shfl_down_sync(0xffffffffu, v.lo, o));
-}
-__device__ __forceinline__ double lu_shfl(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ float lu_shfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ df64 lu_shfl(df64 v, int src) {
-  return df64(__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src));
-}
-// (value, index) maximum over the block; ties go to the smaller index
-template <class R>
-__device__ void lu_block_argmax(R v, int idx, R* wv, int* wi, R& out_v, int& out_i) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    R ov = lu_shfl_down(v, o);
-    int oi = __shfl_down_sync(0xffffffffu, idx, o);
-    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-  }
-  if (lane == 0) { wv[warp] = v; wi[warp] = idx; }
-  __syncthreads();
-  if (warp == 0) {
-    v = lane < nw ? wv[lane] : R(-1.0);
-    idx = lane < nw ? wi[lane] : 0x7fffffff;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      R ov = lu_shfl_down(v, o);
-      int oi = __shfl_down_sync(0xffffffffu, idx, o);
-      if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-    }
-    if (lane == 0) { wv[0] = v; wi[0] = idx; }
-  }
-  __syncthreads();
-  out_v = wv[0]; out_i = wi[0];
-  __syncthreads();
-}
-}  // namespace
-
-template <class R>
-__global__ void __launch_bounds__(LU_PANEL_THREADS) lu_panel_kernel(
-    Cx<R>* __restrict__ Aall, int n, int lda, long long a_bs, int* __restrict__ ipiv_all, long long piv_bs,
-    int32_t* __restrict__ status, int st_div, int k0, int kb) {
-  using C_ = Cx<R>;
-  __shared__ R wv[32];
-  __shared__ int wi[32];
-  __shared__ C_ prow[LU_PB];
-  C_* A = Aall + blockIdx.x * a_bs;
-  int* ipiv = ipiv_all + (long long)blockIdx.x * piv_bs;
-  int32_t* st = status ? status + blockIdx.x / st_div : nullptr;
-  const int tid = threadIdx.x;
-  auto a = [&](int i, int j) -> C_& { return A[i + (long long)j * lda]; };
-  for (int j = k0; j < k0 + kb; ++j) {
-    R best = R(-1.0); int bi = j;
-    for (int i = j + tid; i < n; i += blockDim.x) {
-      const R v = cxabs1(a(i, j));
-      if (v > best) { best = v; bi = i; }
-    }
-    R pv; int p;
-    lu_block_argmax<R>(best, bi, wv, wi, pv, p);
-    if (tid == 0) ipiv[j] = p;
-    // swap rows j, p inside the panel; the pivot row to shared memory
-    if (tid < kb) {
-      const int c = k0 + tid;
-      C_ x = a(j, c), y = a(p, c);
-      if (p != j) { a(j, c) = y; a(p, c) = x; }
-      prow[tid] = (p != j) ? y : x;
-    }
-    __syncthreads();
-    const C_ piv = prow[j - k0];
-    if (piv.x == R(0.0) && piv.y == R(0.0)) {
-      if (tid == 0) wb_flag(st, WB_ST_SINGULAR);
-      continue;
-    }
-    const C_ rp = cxinv(piv);
-    const int ce = k0 + kb;
-    for (int i = j + 1 + tid; i < n; i += blockDim.x) {
-      const C_ l = a(i, j) * rp;
-      a(i, j) = l;
-      for (int c0 = j + 1; c0 < ce; c0 += 8) {
-        C_ v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (c0 + u < ce) v[u] = a(i, c0 + u);
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (c0 + u < ce) a(i, c0 + u) = v[u] - l * prow[c0 + u - k0];
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// One thread per column c outside the panel [k0, k0 + kb): the panel's row swaps in order, and
-// for trailing columns U12 = L11^-1 A12 (L11 unit lower, from shared memory).
-template <class R>
-__global__ void __launch_bounds__(256) lu_swap_trsm_kernel(Cx<R>* __restrict__ Aall, int n, int lda, long long a_bs,
-                                                           const int* __restrict__ ipiv_all, long long piv_bs, int k0,
-                                                           int kb) {
-  using C_ = Cx<R>;
-  __shared__ C_ sL[LU_PB][LU_PB + 1];
-  __shared__ int sp[LU_PB];
-  C_* A = Aall + blockIdx.y * a_bs;
-  const int* ipiv = ipiv_all + (long long)blockIdx.y * piv_bs;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < kb * kb; e += blockDim.x) {
-    const int r = e % kb, c = e / kb;
-    sL[r][c] = A[k0 + r + (long long)(k0 + c) * lda];
-  }
-  if (tid < kb) sp[tid] = ipiv[k0 + tid];
-  __syncthreads();
-  int c = blockIdx.x * blockDim.x + tid;
-  if (c >= n - kb) return;
-  if (c >= k0) c += kb;                      // skip the panel
-  C_* col = A + (long long)c * lda;
-  for (int j = 0; j < kb; ++j) {
-    const int p = sp[j];
-    if (p != k0 + j) {
-      const C_ x = col[k0 + j], y = col[p];
-      col[k0 + j] = y; col[p] = x;
-    }
-  }
-  if (c < k0) return;
-  C_ x[LU_PB];
-#pragma unroll
-  for (int r = 0; r < LU_PB; ++r)
-    if (r < kb) x[r] = col[k0 + r];
-#pragma unroll
-  for (int r = 1; r < LU_PB; ++r) {
-    if (r >= kb) break;
-    C_ acc = x[r];
-#pragma unroll
-    for (int t = 0; t < LU_PB; ++t)
-      if (t < r) acc = acc - sL[r][t] * x[t];
-    x[r] = acc;
-  }
-#pragma unroll
-  for (int r = 1; r < LU_PB; ++r)
-    if (r < kb) col[k0 + r] = x[r];
-}
+constexpr int LU_PB = tri::kPB;        // panel width
 
 // A22 -= L21 U12 on rows and columns [c0, n), K = kb <= LU_PB
 template <class R>
@@ -673,29 +532,70 @@ __global__ void __launch_bounds__(256) lu_update_kernel(Cx<R>* __restrict__ Aall
     }
 }
 
+// CTAs a matrix (a cluster) for a panel of m rows, and its shape. The panel sits in the CTAs' shared
+// memory, so C is at least what that takes. FP32: one CTA if it holds the panel, a column costs latency
+// (barriers, a reciprocal) and a cluster's barrier costs more of it: 93 -> 30 us a panel of 450 rows. FP64:
+// a row's update is FP64 issue, so up to 8 CTAs while the batch leaves SMs idle: 600 -> 100 us.
+struct PanelShape { int ctas, rows, threads, slices; size_t smem; };
+template <class R> static PanelShape panel_shape(int batch, int m, int kb) {
+  PanelShape p;
+  const size_t row = (size_t)kb * sizeof(Cx<R>), most = 212 * 1024;
+  int c = 1;
+  while (c < tri::kPanelMaxCluster && (size_t)((m + c - 1) / c) * row > most) c *= 2;
+  if (std::is_same<R, double>::value)
+    while (2 * c <= tri::kPanelMaxCluster && 2LL * c * batch <= sm_count() && (m + 2 * c - 1) / (2 * c) >= 24) c *= 2;
+  p.ctas = c;
+  p.rows = (m + c - 1) / c;
+  p.threads = p.rows <= 64 ? 256 : tri::kPanelThreads;
+  p.slices = 1;
+  while (p.slices < 8 && 2 * p.slices * p.rows <= p.threads) p.slices *= 2;
+  p.smem = p.rows * row;
+  return p;
+}
+
 template <class R>
 void getrf(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a_bs, int* ipiv, long long piv_bs,
            int32_t* status, int st_div) {
   if (batch <= 0 || n <= 0) return;
   st_div = st_div < 1 ? 1 : st_div;
-  if (batch >= 2 * sm_count() || n < 2 * LU_PB) {
+  // One CTA a matrix: FP32 and double-float batches that fill the GPU so, and what a panel or two would
+  // cover. FP64 takes the panels from the second one on, whatever the batch: its updates run on the
+  // tensor cores there, on the FP64 pipes here (n = 50: 830 -> 230 us).
+  constexpr bool fp64 = std::is_same<R, double>::value;
+  if (fp64 ? n <= LU_PB : (batch >= 2 * sm_count() || n < 2 * LU_PB)) {
     getrf_kernel<R><<<batch, LU_THREADS, 0, s>>>(A, n, lda, a_bs, ipiv, piv_bs, status, st_div);
     note_launch();
     return;
   }
-  for (int k0 = 0; k0 < n; k0 += LU_PB) {
-    const int kb = min(LU_PB, n - k0);
-    lu_panel_kernel<R><<<batch, LU_PANEL_THREADS, 0, s>>>(A, n, lda, a_bs, ipiv, piv_bs, status, st_div, k0, kb);
+  int width = LU_PB;
+  while (width > 8 && panel_shape<R>(batch, n, width).smem > 212 * 1024) width /= 2;
+  cudaFuncSetAttribute(tri::lu_panel_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024);
+  for (int k0 = 0; k0 < n; k0 += width) {
+    const int kb = min(width, n - k0);
+    const PanelShape sh = panel_shape<R>(batch, n - k0, kb);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(batch * sh.ctas));
+    cfg.blockDim = dim3((unsigned)sh.threads);
+    cfg.dynamicSmemBytes = sh.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)sh.ctas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, tri::lu_panel_kernel<R>, A, n, lda, a_bs, ipiv, piv_bs, status, st_div, k0, kb, sh.rows,
+                       sh.slices);
     note_launch();
     if (n - kb > 0) {
-      dim3 g2((n - kb + 255) / 256, batch);
-      lu_swap_trsm_kernel<R><<<g2, 256, 0, s>>>(A, n, lda, a_bs, ipiv, piv_bs, k0, kb);
+      dim3 g2((n - kb + tri::kSwapThreads / 8 - 1) / (tri::kSwapThreads / 8), batch);
+      tri::lu_swap_trsm_kernel<R><<<g2, tri::kSwapThreads, 0, s>>>(A, n, lda, a_bs, ipiv, piv_bs, k0, kb);
       note_launch();
     }
     const int m = n - k0 - kb;
     if (m > 0) {
       const int c0 = k0 + kb;
-      if constexpr (std::is_same<R, double>::value) {   // A22 -= L21 U12
+      if constexpr (fp64) {   // A22 -= L21 U12
         if (oz_zgemm(s, batch, m, m, kb, make_double2(-1.0, 0.0), (const cplx*)A + c0 + (long long)k0 * lda, 1, lda,
                      a_bs, nullptr, false, (const cplx*)A + k0 + (long long)c0 * lda, 1, lda, a_bs, false,
                      make_double2(1.0, 0.0), (cplx*)A + c0 + (long long)c0 * lda, 1, lda, a_bs))
@@ -836,219 +736,78 @@ __global__ void __launch_bounds__(256) getrs_kernel(
   }
 }
 
-// Few right-hand sides (the cascade's incidence columns): one CTA per matrix holds X = B
-// (n x NC) in shared memory and substitutes 32 rows at a time. Per block: the 32 x 32 diagonal
-// block is staged in shared memory, warp 0 solves it with the block's rows in its lanes
-// (shuffles carry each solved row to the others), then every thread takes rows below (above,
-// going back) and subtracts the block's contribution, reading L (U) down its columns, coalesced.
-constexpr int NS_B = 32;
-constexpr int NS_THREADS = 1024;
-
-template <class R, int NC>
-__global__ void __launch_bounds__(NS_THREADS) getrs_narrow_kernel(
-    const Cx<R>* __restrict__ LUall, int n, int lda, long long a_bs, const int* __restrict__ ipiv_all,
-    long long piv_bs, Cx<R>* __restrict__ Ball, int nrhs, int ldb, long long b_bs) {
-  using C_ = Cx<R>;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  C_* X = reinterpret_cast<C_*>(smraw);            // (n, NC), row-major
-  __shared__ C_ sD[NS_B][NS_B + 1];
-  const C_* LU = LUall + blockIdx.x * a_bs;
-  const int* ipiv = ipiv_all + (long long)blockIdx.x * piv_bs;
-  C_* B = Ball + blockIdx.x * b_bs;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < n * NC; e += blockDim.x) {
-    const int r = e % n, c = e / n;
-    X[r * NC + c] = (c < nrhs) ? B[r + (long long)c * ldb] : cxzero<R>();
-  }
-  __syncthreads();
-  if (tid < nrhs) {                                // the row swaps, in order, one column each
-    for (int j = 0; j < n; ++j) {
-      const int p = ipiv[j];
-      if (p != j) { const C_ t = X[j * NC + tid]; X[j * NC + tid] = X[p * NC + tid]; X[p * NC + tid] = t; }
-    }
-  }
-  for (int sweep = 0; sweep < 2; ++sweep) {
-    const bool fwd = sweep == 0;                   // L (unit lower), then U (upper)
-    const int nblk = (n + NS_B - 1) / NS_B;
-    for (int bi = 0; bi < nblk; ++bi) {
-      const int i0 = fwd ? bi * NS_B : max(0, n - (bi + 1) * NS_B);
-      const int ib = fwd ? min(NS_B, n - i0) : (n - bi * NS_B) - i0;
-      __syncthreads();
-      for (int e = tid; e < NS_B * NS_B; e += blockDim.x) {
-        const int r = e % NS_B, c = e / NS_B;
-        sD[r][c] = (r < ib && c < ib) ? LU[i0 + r + (long long)(i0 + c) * lda] : cxzero<R>();
-      }
-      __syncthreads();
-      if (warp == 0) {
-        C_ x[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) x[c] = lane < ib ? X[(i0 + lane) * NC + c] : cxzero<R>();
-        if (fwd) {
-          for (int t = 0; t < ib; ++t) {
-            const C_ l = sD[lane][t];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-              C_ xt;
-              xt.x = lu_shfl(x[c].x, t);
-              xt.y = lu_shfl(x[c].y, t);
-              if (lane > t) x[c] = x[c] - l * xt;
-            }
-          }
-        } else {
-          for (int t = ib - 1; t >= 0; --t) {
-            if (lane == t) {
-              const C_ d = sD[t][t];
-#pragma unroll
-              for (int c = 0; c < NC; ++c) x[c] = cxdiv(x[c], d);
-            }
-            const C_ u = sD[lane][t];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-              C_ xt;
-              xt.x = lu_shfl(x[c].x, t);
-              xt.y = lu_shfl(x[c].y, t);
-              if (lane < t) x[c] = x[c] - u * xt;
-            }
-          }
-        }
-        if (lane < ib) {
-#pragma unroll
-          for (int c = 0; c < NC; ++c) X[(i0 + lane) * NC + c] = x[c];
-        }
-      }
-      __syncthreads();
-      // the block's contribution to the rows still to solve
-      const int rs = fwd ? i0 + ib : 0, re = fwd ? n : i0;
-      for (int i = rs + tid; i < re; i += blockDim.x) {
-        C_ acc[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] = X[i * NC + c];
-        const C_* li = LU + i + (long long)i0 * lda;
-        for (int t = 0; t < ib; ++t) {
-          const C_ l = li[(long long)t * lda];
-#pragma unroll
-          for (int c = 0; c < NC; ++c) acc[c] = acc[c] - l * X[(i0 + t) * NC + c];
-        }
-#pragma unroll
-        for (int c = 0; c < NC; ++c) X[i * NC + c] = acc[c];
-      }
-    }
-  }
-  __syncthreads();
-  for (int e = tid; e < n * nrhs; e += blockDim.x) {
-    const int r = e % n, c = e / n;
-    B[r + (long long)c * ldb] = X[r * NC + c];
-  }
-}
-
+// Few right-hand sides (the cascade's incidence columns), by a cluster a matrix (tri::getrs_narrow_kernel).
+// FP32 is bound by the diagonal blocks' chains and needs a second CTA only for its loads' sake; FP64's
+// updates are FP64 issue. 3 columns at n = 450: FP64 3.0 -> 0.4 ms, FP32 6 columns 1.0 -> 0.2 ms.
 template <class R, int NC>
 static bool getrs_narrow(cudaStream_t s, int batch, int n, const Cx<R>* LU, int lda, long long a_bs, const int* ipiv,
                          long long piv_bs, Cx<R>* B, int nrhs, int ldb, long long b_bs) {
-  const size_t sm = (size_t)n * NC * sizeof(Cx<R>);
-  if (sm > (size_t)200 * 1024) return false;
-  cudaFuncSetAttribute(getrs_narrow_kernel<R, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  getrs_narrow_kernel<R, NC><<<batch, NS_THREADS, sm, s>>>(LU, n, lda, a_bs, ipiv, piv_bs, B, nrhs, ldb, b_bs);
+  const size_t sm = (size_t)n * (NC * sizeof(Cx<R>) + 2 * sizeof(int));
+  if (sm > (size_t)180 * 1024) return false;
+  const int want = std::is_same<R, double>::value ? (n < 64 ? 1 : n < 128 ? 2 : n < 256 ? 4 : 8)
+                                                  : (n < 480 ? 1 : n < 960 ? 2 : 4);
+  int c = 1;
+  while (2 * c <= want && 2LL * c * batch <= sm_count()) c *= 2;
+  cudaFuncSetAttribute(tri::getrs_narrow_kernel<R, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(batch * c));
+  cfg.blockDim = dim3((unsigned)(n <= 128 ? 256 : tri::kNarrowThreads));
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)c;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, tri::getrs_narrow_kernel<R, NC>, LU, n, lda, a_bs, ipiv, piv_bs, B, nrhs, ldb, b_bs);
   note_launch();
   return true;
 }
 
-// Many right-hand sides: a blocked substitution across the GPU. The FP32 form's cascade always
-// takes it; FP64 takes it only for batches too small to fill the GPU with getrs_kernel's CTAs
-// (stage A's outer inverses: a few N x N systems with N right-hand sides), since a large FP64
-// batch is bound by FP64 issue either way.
-// The row interchanges are applied first (trans 0) or last (trans 1), one thread per column;
-// then, per block of TB_NB rows, trsm_diag_kernel solves the diagonal block for every column
-// (the block and 64 columns in shared memory, one thread per column) and the batched GEMM
-// subtracts the block's contribution from the rows still to solve (K = TB_NB). The
-// substitution order and pivots are those of getrs_kernel; only the summation order differs.
-constexpr int TB_NB = 64;
-constexpr int TB_W = 64;
-
-template <class R>
-__global__ void laswp_kernel(Cx<R>* __restrict__ Ball, int n, int nrhs, int ldb, long long b_bs,
-                             const int* __restrict__ ipiv_all, long long piv_bs, int forward) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nrhs) return;
-  Cx<R>* col = Ball + blockIdx.y * b_bs + (long long)c * ldb;
-  const int* ipiv = ipiv_all + (long long)blockIdx.y * piv_bs;
-  if (forward) {
-    for (int j = 0; j < n; ++j) {
-      const int p = ipiv[j];
-      if (p != j) { const Cx<R> t = col[j]; col[j] = col[p]; col[p] = t; }
-    }
-  } else {
-    for (int j = n - 1; j >= 0; --j) {
-      const int p = ipiv[j];
-      if (p != j) { const Cx<R> t = col[j]; col[j] = col[p]; col[p] = t; }
-    }
-  }
-}
-
-// op(A)'s diagonal block [i0, i0 + ib) solved for TB_W columns: lower (forward) or upper
-// (backward) triangle, unit or stored diagonal; op(A) = A (trans 0) or A^T (trans 1).
-template <class R>
-__global__ void __launch_bounds__(TB_W) trsm_diag_kernel(const Cx<R>* __restrict__ LUall, int lda, long long a_bs,
-                                                         Cx<R>* __restrict__ Ball, int nrhs, int ldb, long long b_bs,
-                                                         int i0, int ib, int lower, int unit, int trans) {
-  using C_ = Cx<R>;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  C_* sL = reinterpret_cast<C_*>(smraw);                 // (TB_NB, TB_NB + 1)
-  C_* sX = sL + TB_NB * (TB_NB + 1);                     // (TB_NB, TB_W + 1)
-  const C_* LU = LUall + blockIdx.y * a_bs;
-  C_* B = Ball + blockIdx.y * b_bs;
-  const int c0 = blockIdx.x * TB_W, tid = threadIdx.x;
-  const int w = min(TB_W, nrhs - c0);
-  for (int e = tid; e < TB_NB * TB_NB; e += blockDim.x) {
-    const int r = e % TB_NB, t = e / TB_NB;
-    C_ v = cxzero<R>();
-    if (r < ib && t < ib) v = trans ? LU[i0 + t + (long long)(i0 + r) * lda] : LU[i0 + r + (long long)(i0 + t) * lda];
-    sL[r * (TB_NB + 1) + t] = v;
-  }
-  for (int e = tid; e < TB_NB * TB_W; e += blockDim.x) {
-    const int r = e % TB_NB, c = e / TB_NB;
-    sX[r * (TB_W + 1) + c] = (r < ib && c < w) ? B[i0 + r + (long long)(c0 + c) * ldb] : cxzero<R>();
-  }
-  __syncthreads();
-  if (tid < w) {
-    auto L = [&](int r, int t) -> C_ { return sL[r * (TB_NB + 1) + t]; };
-    auto X = [&](int r) -> C_& { return sX[r * (TB_W + 1) + tid]; };
-    if (lower) {
-      for (int r = 0; r < ib; ++r) {
-        C_ acc = X(r);
-        for (int t = 0; t < r; ++t) acc = acc - L(r, t) * X(t);
-        if (!unit) acc = cxdiv(acc, L(r, r));
-        X(r) = acc;
-      }
-    } else {
-      for (int r = ib - 1; r >= 0; --r) {
-        C_ acc = X(r);
-        for (int t = r + 1; t < ib; ++t) acc = acc - L(r, t) * X(t);
-        if (!unit) acc = cxdiv(acc, L(r, r));
-        X(r) = acc;
-      }
-    }
-  }
-  __syncthreads();
-  for (int e = tid; e < TB_NB * TB_W; e += blockDim.x) {
-    const int r = e % TB_NB, c = e / TB_NB;
-    if (r < ib && c < w) B[i0 + r + (long long)(c0 + c) * ldb] = sX[r * (TB_W + 1) + c];
-  }
-}
+// Many right-hand sides: a blocked substitution across the GPU. The FP32 form's cascade and the FP64
+// form take it, the latter with its products on the tensor cores.
+// The row interchanges are applied first (trans 0) or last (trans 1); then, per block of TB_NB rows, the
+// diagonal block is solved for every column (tri::trsm_diag_kernel, in FP32's upper solve
+// trsm_upper_f32_kernel) and the batched GEMM subtracts the block's contribution from the rows still to
+// solve (K = TB_NB). The substitution order and pivots are those of getrs_kernel; only the summation
+// order differs. A diagonal block of 450 columns: FP64 400 -> 80 us, FP32 65 -> 20 us.
+constexpr int TB_NB = tri::kTB;
 
 template <class R>
 static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int lda, long long a_bs, const int* ipiv,
                           long long piv_bs, Cx<R>* B, int nrhs, int ldb, long long b_bs, int trans) {
-  const dim3 gs((nrhs + 127) / 128, batch);
-  if (trans == 0) { laswp_kernel<R><<<gs, 128, 0, s>>>(B, n, nrhs, ldb, b_bs, ipiv, piv_bs, 1); note_launch(); }
-  const size_t sm = sizeof(Cx<R>) * ((size_t)TB_NB * (TB_NB + 1) + (size_t)TB_NB * (TB_W + 1));
-  cudaFuncSetAttribute(trsm_diag_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  const dim3 gd((nrhs + TB_W - 1) / TB_W, batch);
+  // interchanges: a few columns a CTA, so that about two CTAs an SM run
+  const size_t smp = (size_t)n * (sizeof(Cx<R>) + 2 * sizeof(int));
+  const int cols = max(1, (int)((long long)nrhs * batch / (4LL * sm_count())));
+  const dim3 gs((nrhs + cols - 1) / cols, batch);
+  cudaFuncSetAttribute(tri::laswp_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smp);
+  if (trans == 0) {
+    tri::laswp_kernel<R><<<gs, 256, smp, s>>>(B, n, nrhs, ldb, b_bs, ipiv, piv_bs, 1, cols);
+    note_launch();
+  }
+  const size_t sm = sizeof(Cx<R>) * (size_t)TB_NB * (TB_NB + 1);
+  cudaFuncSetAttribute(tri::trsm_diag_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const dim3 gd((nrhs + tri::kTriThreads / 8 - 1) / (tri::kTriThreads / 8), batch);
+  auto diagonal = [&](int i0, int ib, int lower, int unit) {
+    if constexpr (sizeof(R) == 4) {
+      if (!lower) {
+        const size_t su = sizeof(Cx<R>) * (size_t)(TB_NB + 32) * (TB_NB + 1);
+        cudaFuncSetAttribute(tri::trsm_upper_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su);
+        tri::trsm_upper_f32_kernel<<<dim3((nrhs + 31) / 32, batch), 32, su, s>>>(
+            (const Cx<float>*)LU, lda, a_bs, (Cx<float>*)B, nrhs, ldb, b_bs, i0, ib, unit, trans);
+        note_launch();
+        return;
+      }
+    }
+    tri::trsm_diag_kernel<R><<<gd, tri::kTriThreads, sm, s>>>(LU, lda, a_bs, B, nrhs, ldb, b_bs, i0, ib, lower, unit, trans);
+    note_launch();
+  };
   const double2 m1 = make_double2(-1.0, 0.0), p1 = make_double2(1.0, 0.0);
   // forward: L (unit lower) for trans 0, U^T (lower, stored diagonal) for trans 1
   for (int i0 = 0; i0 < n; i0 += TB_NB) {
     const int ib = min(TB_NB, n - i0), i1 = i0 + ib, m = n - i1;
-    trsm_diag_kernel<R><<<gd, TB_W, sm, s>>>(LU, lda, a_bs, B, nrhs, ldb, b_bs, i0, ib, 1, trans == 0, trans);
-    note_launch();
+    diagonal(i0, ib, 1, trans == 0);
     if (m > 0) {
       if (trans == 0)
         gemm<R>(s, batch, m, nrhs, ib, m1, LU + i1 + (long long)i0 * lda, 1, lda, a_bs, B + i0, 1, ldb, b_bs, p1,
@@ -1061,8 +820,7 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
   // backward: U (upper, stored diagonal) for trans 0, L^T (unit upper) for trans 1
   for (int i1 = n; i1 > 0; i1 -= TB_NB) {
     const int i0 = max(0, i1 - TB_NB), ib = i1 - i0;
-    trsm_diag_kernel<R><<<gd, TB_W, sm, s>>>(LU, lda, a_bs, B, nrhs, ldb, b_bs, i0, ib, 0, trans == 1, trans);
-    note_launch();
+    diagonal(i0, ib, 0, trans == 1);
     if (i0 > 0) {
       if (trans == 0)
         gemm<R>(s, batch, i0, nrhs, ib, m1, LU + (long long)i0 * lda, 1, lda, a_bs, B + i0, 1, ldb, b_bs, p1, B, 1,
@@ -1071,7 +829,10 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
         gemm<R>(s, batch, i0, nrhs, ib, m1, LU + i0, lda, 1, a_bs, B + i0, 1, ldb, b_bs, p1, B, 1, ldb, b_bs);
     }
   }
-  if (trans == 1) { laswp_kernel<R><<<gs, 128, 0, s>>>(B, n, nrhs, ldb, b_bs, ipiv, piv_bs, 0); note_launch(); }
+  if (trans == 1) {
+    tri::laswp_kernel<R><<<gs, 256, smp, s>>>(B, n, nrhs, ldb, b_bs, ipiv, piv_bs, 0, cols);
+    note_launch();
+  }
 }
 
 template <class R>
@@ -1082,12 +843,14 @@ void getrs(cudaStream_t s, int batch, int n, const Cx<R>* LU, int lda, long long
     getrs_blocked<R>(s, batch, n, LU, lda, a_bs, ipiv, piv_bs, B, nrhs, ldb, b_bs, trans);
     return;
   }
-  if (std::is_same<R, double>::value && nrhs >= 2 * SV_W && n >= 2 * TB_NB &&
-      (long long)batch * ((nrhs + SV_W - 1) / SV_W) < sm_count()) {
-    getrs_blocked<R>(s, batch, n, LU, lda, a_bs, ipiv, piv_bs, B, nrhs, ldb, b_bs, trans);
-    return;
+  constexpr bool fp64 = std::is_same<R, double>::value;
+  if constexpr (fp64) {          // FP64: from 8 columns on (n = 50: 580 -> 110 us)
+    if (nrhs >= 8) {
+      getrs_blocked<R>(s, batch, n, LU, lda, a_bs, ipiv, piv_bs, B, nrhs, ldb, b_bs, trans);
+      return;
+    }
   }
-  if (trans == 0 && n >= 64 && batch < 4 * sm_count()) {
+  if (trans == 0 && (fp64 || (n >= 64 && batch < 4 * sm_count()))) {
     if (nrhs <= 3 && getrs_narrow<R, 3>(s, batch, n, LU, lda, a_bs, ipiv, piv_bs, B, nrhs, ldb, b_bs)) return;
     if (nrhs > 3 && nrhs <= 6 && getrs_narrow<R, 6>(s, batch, n, LU, lda, a_bs, ipiv, piv_bs, B, nrhs, ldb, b_bs))
       return;
