@@ -38,6 +38,7 @@
 // 2 layers at orders (5, 5) 671 -> 412 ms; at n = 1250 and one matrix per SM the far updates' memory
 // traffic (2 (2n - 2) complex values a reflector) is next.
 #pragma once
+#include <type_traits>
 #include "wb_common.cuh"
 #include "wb_num.cuh"
 
@@ -671,6 +672,228 @@ __device__ __noinline__ void chase_window(Cx<R>* H, int ldh, const Cx<R>* tile, 
   __syncwarp();
 }
 
+// FP64: an instruction takes 64 cycles of a warp's issue on GB300 whatever its active lanes, so the
+// elements are spread over the lanes by their real components. For the left application lane 4 j + c
+// carries component c of column k + j's pair (c = 0, 1: row k; 2, 3: row k + 1), 8 columns a set, the
+// window's columns in up to three sets that move down a slot a step; for the right one lane 4 r + c
+// carries row k - 1 + r of columns k, k + 1. Each application is then three operations
+// (cx u + (+-cy) v + (+-s) w, the partners v and w by shuffles) instead of twelve, in the order of
+// left_pair and right_pair: the bits are theirs.
+__device__ __forceinline__ double flip(double v, int mask) {    // v with its sign changed by mask (0 or 1 << 31)
+  return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
+}
+__device__ __forceinline__ double shx(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
+
+// 1 / sqrt(v) to 22 bits for normal v > 0, from the FP32 unit; the exponents by integer operations
+// (a conversion costs as much as an FP64 operation).
+__device__ __forceinline__ double rsqrt_start(double v) {
+  int hi = __double2hiint(v);
+  const int k = ((hi >> 20) - 1023) & ~1;
+  hi -= k * (1 << 20);                                          // v / 2^k in [1, 4)
+  float f = __int_as_float((int)(((unsigned)(hi - (896 << 20)) << 3) | ((unsigned)__double2loint(v) >> 29)));
+  asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(f));
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double((int)(b >> 3) + (896 - (k >> 1)) * (1 << 20), (int)(b << 29));
+}
+
+struct Chase64 {
+  double L[3];                 // left layout: this lane's component of its pair in every set
+  double eu, ev, ew;           // right layout, rows k - 1 and k + 2: the component and its partners
+  double cx, cy, s;            // the rotation
+};
+
+template <int NS>
+__device__ __forceinline__ void chase64_step(Chase64& v, Cx<double>* H, int ldh, const double* tile, int q, int k0, int o,
+                                             int i, int cmax, bool lastw, QrRecord<double>& g, uint64_t* bars) {
+  constexpr int MW = QrWin<double>::m, TL = QrTile<double>::ld;
+  const int lane = threadIdx.x & 31, c = lane & 3, slot = lane >> 2, k = k0 + q;
+  const int left = (c == 1 || c == 2) ? 1 << 31 : 0, rest = c >= 2 ? 1 << 31 : 0;
+  const int col2 = (c >> 1) * 4 + (c & 1);                      // row k of column k + c / 2
+  if (lane < 2) reinterpret_cast<double*>(&g.t1[q])[lane] = lane ? v.cy : v.cx;
+  if (lane == 2) g.t2[q] = v.s;
+  // the rows the next step needs: row k + 2 of the columns, (k + 3, k + 2)
+  double nb[NS];
+#pragma unroll
+  for (int t = 0; t < NS; ++t) {
+    const int jj = q - 1 + 8 * t + slot;
+    const bool in = jj >= 0 && jj < MW && k0 + 2 + jj <= cmax;
+    nb[t] = in ? tile[2 * (jj * TL + o + q + 2) + (c & 1)] : 0.0;
+  }
+  const double n21x = tile[2 * (q * TL + o + q + 3)], n21y = tile[2 * (q * TL + o + q + 3) + 1];
+  // left on columns k ..
+  const double cyl = flip(v.cy, left), sl = flip(v.s, rest);
+  double Ln[NS];
+#pragma unroll
+  for (int t = 0; t < NS; ++t) Ln[t] = fma(v.cx, v.L[t], fma(cyl, shx(v.L[t], 1), sl * shx(v.L[t], 2)));
+  // right on rows k - 1 .. k + 2 of columns k, k + 1; lane 16 makes the square of (k + 2, k)
+  double u = shf(Ln[0], (lane & 8 ? 2 : 0) + col2), pv = shf(Ln[0], ((lane & 8 ? 2 : 0) + col2) ^ 1);
+  double pw = shf(Ln[0], ((lane & 8 ? 2 : 0) + col2) ^ 4);
+  if (slot != 1 && slot != 2) { u = v.eu; pv = v.ev; pw = v.ew; }
+  const double r1 = sl * pw;
+  const bool sq = slot == 4;
+  const double r2 = fma(sq ? r1 : flip(cyl, 1 << 31), sq ? r1 : pv, sq ? 0.0 : r1);
+  const double Rn = fma(v.cx, u, r2);
+  const double ax = shf(Rn, 8), ay = shf(Rn, 9), xx = shf(Rn, 12), x2 = shf(Rn, 16);
+  // the finished row k of the columns past k + 2
+#pragma unroll
+  for (int t = 0; t < NS; ++t) {
+    const int col = k + 8 * t + slot;
+    if (c < 2 && 8 * t + slot >= 3 && col <= cmax) reinterpret_cast<double*>(H + k + (long long)col * ldh)[c] = Ln[t];
+  }
+  double subx = ax, suby = ay;
+  double top = Rn;                                              // what the band keeps, right layout
+  if (k + 1 < i) {
+    const int e = max(max(__double2hiint(ax) & 0x7fffffff, __double2hiint(ay) & 0x7fffffff), __double2hiint(xx) & 0x7fffffff) >> 20;
+    if (e < 1023 - 400 || e > 1023 + 400 || (xx == 0.0 && ay == 0.0)) {
+      const Rot<double> rn = chase_reflector<double>(cxmk<double>(ax, ay), xx);
+      if (!rn.identity) { subx = rn.beta; suby = 0.0; }
+      v.cx = rn.t1.x; v.cy = rn.t1.y; v.s = rn.t2;
+    } else {
+      // (ax, ay, xx, ss) / sqrt(ss), one a lane, by one third-order step from a 22-bit start
+      const double ss = fma(ax, ax, fma(ay, ay, x2)), y = rsqrt_start(ss);
+      const double z = (c == 0 ? ax : c == 1 ? ay : c == 2 ? xx : ss) * y;
+      const double d = fma(-shf(z, 3), y, 1.0);
+      const double res = fma(z, d * fma(d, 0.375, 0.5), z);
+      v.cx = shf(res, 0); v.cy = shf(res, 1); v.s = shf(res, 2);
+      subx = shf(res, 3); suby = 0.0;
+    }
+    // the pairs of step k + 1
+    double m[NS];
+#pragma unroll
+    for (int t = 0; t < NS; ++t) m[t] = shf(Ln[t], (lane + 6) & 31);
+    const double core = shf(Rn, 10 + (c & 1) + 4 * (c >> 1));
+#pragma unroll
+    for (int t = 0; t < NS; ++t) v.L[t] = c >= 2 ? nb[t] : slot < 7 ? m[t] : t + 1 < NS ? m[t + 1 < NS ? t + 1 : t] : 0.0;
+    if (slot == 0) v.L[0] = core;
+    const double xn = shf(Rn, 6 + (c & 1)), yn = shf(Ln[0], 8 + (c & 1));
+    const double xo = shx(xn, 1), yo = shx(yn, 1);
+    v.eu = slot == 0 ? (c < 2 ? xn : yn) : 0.0;
+    v.ev = slot == 0 ? (c < 2 ? xo : yo) : 0.0;
+    v.ew = slot == 0 ? (c < 2 ? yn : xn) : c == 0 ? n21x : c == 1 ? n21y : 0.0;
+    if (slot == 3 && c >= 2) { v.eu = c == 2 ? n21x : n21y; v.ev = c == 2 ? n21y : n21x; }
+  } else {
+    // the sweep's last subdiagonal made real; the factor goes to column k + 1
+    Cx<double> sc = cxone<double>();
+    int scaled = 0;
+    if (ay != 0.0) {
+      const double am = modulus(cxmk<double>(ax, ay));
+      if (am > RealT<double>::tiny()) {
+        subx = am; suby = 0.0;
+        sc = cxmk<double>(ax, ay) * (1.0 / am);
+        scaled = 1;
+      } else {
+        suby = 0.0;
+      }
+    }
+    const double other = shx(Rn, 1);
+    if (scaled && c >= 2 && slot <= 1) {
+      const Cx<double> p = c == 2 ? cxmk<double>(Rn, other) : cxmk<double>(other, Rn);
+      const Cx<double> w = sc * p;
+      top = c == 2 ? w.x : w.y;
+    }
+    if (lane == 0) { g.sc = sc; g.scaled = scaled; }
+    if (c >= 2 && (slot == 1 || slot == 2)) reinterpret_cast<double*>(H + (i - 2 + slot) + (long long)i * ldh)[c - 2] = top;
+  }
+  if (slot == 2 && c < 2) top = c ? suby : subx;
+  if (slot < 3 && (slot == 0 || c < 2) && (slot > 0 || k > 0))
+    reinterpret_cast<double*>(H + (k - 1 + slot) + (long long)(k + (c >> 1)) * ldh)[c & 1] = top;
+  __syncwarp();
+  if (!lastw && (q + 1) % kQrStride == 0 && lane == 0) publish(bars, q / kQrStride);
+}
+
+__device__ __noinline__ void chase_window64(Cx<double>* H, int ldh, const Cx<double>* tile, const Request& rq,
+                                            QrChase<double>& cs, QrRecord<double>& g, uint64_t* bars) {
+  constexpr int MW = QrWin<double>::m, TL = QrTile<double>::ld;
+  static_assert(MW + 2 <= 24, "three sets of columns");
+  __builtin_assume(__isShared(tile)); __builtin_assume(__isShared(&cs)); __builtin_assume(__isShared(&g));
+  const int lane = threadIdx.x & 31, c = lane & 3, slot = lane >> 2;
+  const int i = rq.i, k0 = rq.k0, k1 = rq.k1, o = k0 - rq.base, cmax = min(k1 + 1, i);
+  const bool lastw = k1 == i;
+  const double* td = reinterpret_cast<const double*>(tile);
+  Chase64 v;
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const int jj = 8 * t + slot - 2;
+    v.L[t] = (jj >= 0 && jj < MW && k0 + 2 + jj <= cmax) ? td[2 * (jj * TL + o + (c >> 1)) + (c & 1)] : 0.0;
+  }
+  auto part = [](const Cx<double>& a, int p) { return p ? a.y : a.x; };
+  if (slot == 0) v.L[0] = part(c < 2 ? cs.c00 : cs.c10, c & 1);
+  if (slot == 1) v.L[0] = part(c < 2 ? cs.c01 : cs.c11, c & 1);
+  v.eu = v.ev = v.ew = 0.0;
+  if (slot == 0) {
+    v.eu = part(c < 2 ? cs.x : cs.y, c & 1);
+    v.ev = part(c < 2 ? cs.x : cs.y, (c & 1) ^ 1);
+    v.ew = part(c < 2 ? cs.y : cs.x, c & 1);
+  } else if (c < 2) {
+    v.ew = part(cs.c21, c);
+  } else if (slot == 3) {
+    v.eu = part(cs.c21, c & 1);
+    v.ev = part(cs.c21, (c & 1) ^ 1);
+  }
+  v.cx = cs.t1.x; v.cy = cs.t1.y; v.s = cs.t2;
+  __syncwarp();
+  if (lane == 0) { g.sc = cxone<double>(); g.scaled = 0; }
+  const int nc = cmax - k0 + 1;                                 // columns at the window's first step
+  int q = 0;
+#pragma unroll 1
+  for (; q < k1 - k0 && nc - q > 16; ++q) chase64_step<3>(v, H, ldh, td, q, k0, o, i, cmax, lastw, g, bars);
+#pragma unroll 1
+  for (; q < k1 - k0 && nc - q > 8; ++q) chase64_step<2>(v, H, ldh, td, q, k0, o, i, cmax, lastw, g, bars);
+#pragma unroll 1
+  for (; q < k1 - k0; ++q) chase64_step<1>(v, H, ldh, td, q, k0, o, i, cmax, lastw, g, bars);
+  if (slot < 2) reinterpret_cast<double*>(slot ? (c < 2 ? &cs.c01 : &cs.c11) : (c < 2 ? &cs.c00 : &cs.c10))[c & 1] = v.L[0];
+  if (slot == 0) reinterpret_cast<double*>(c < 2 ? &cs.x : &cs.y)[c & 1] = v.eu;
+  if (slot == 3 && c >= 2) reinterpret_cast<double*>(&cs.c21)[c & 1] = v.eu;
+  if (lane == 0) {
+    const int k2 = min(k1 + MW, i), k3 = min(k2 + MW, i);
+    g.k0 = k0; g.k1 = k1;
+    g.cfar = min(k3 + 1, i) + 1;
+    cs.t1 = cxmk<double>(v.cx, v.cy); cs.v2 = cxzero<double>(); cs.t2 = v.s;
+    if (lastw) { cs.drain = k0; cs.k0 = -1; }
+    else { cs.kp = k0; cs.k0 = k1; cs.base = rq.kp; cs.tile ^= 1; }
+  }
+  __syncwarp();
+}
+
+// The near columns in FP64: warp `part` (0, 1) carries eight of them, four lanes a column as above.
+__device__ __noinline__ bool near_columns64(Cx<double>* H, int ldh, Cx<double>* tile, const Request& rq, int part,
+                                            const QrRecord<double>& g, const QrRecord<double>& gp, uint64_t* bars,
+                                            uint32_t parity) {
+  constexpr int MW = QrWin<double>::m, TL = QrTile<double>::ld;
+  static_assert(MW == 16, "two warps of eight columns");
+  __builtin_assume(__isShared(tile)); __builtin_assume(__isShared(&g)); __builtin_assume(__isShared(&gp));
+  const int lane = threadIdx.x & 31, c = lane & 3, slot = lane >> 2;
+  const int k0 = rq.k0, k1 = rq.k1, kp = rq.kp, i = rq.i;
+  const int k2 = min(k1 + MW, i), c0 = k1 + 2 + 8 * part, cmax = min(min(k2 + 1, i), c0 + 7);
+  tile += 8 * part * TL;
+  load_tile<double>(H, ldh, tile, c0, cmax, kp, k2, i, 0, 1);
+  __syncwarp();
+  const bool mine = c0 + slot <= cmax;
+  double* col = reinterpret_cast<double*>(tile + slot * TL) + (c & 1);
+  double* out = reinterpret_cast<double*>(H + kp + (long long)(c0 + slot) * ldh) + (c & 1);
+  const int left = (c == 1 || c == 2) ? 1 << 31 : 0, rest = c >= 2 ? 1 << 31 : 0;
+  double L = c < 2 ? col[0] : col[2];
+  bool ok = true;
+  const int np = k0 - kp, nt = k1 - kp;
+  for (int r = 0; r < nt; ++r) {
+    const int q = r - np;
+    if (q >= 0 && q % kQrStride == 0) {
+      ok = ok && await(bars, q / kQrStride, parity);
+      __syncwarp();
+    }
+    const QrRecord<double>& gr = q < 0 ? gp : g;
+    const int e = q < 0 ? r : q;
+    const Cx<double> t1 = gr.t1[e];
+    const double s = gr.t2[e], nb = col[2 * (r + 2)];
+    const double Ln = fma(t1.x, L, fma(flip(t1.y, left), shx(L, 1), flip(s, rest) * shx(L, 2)));
+    const double dn = shx(Ln, 2);
+    if (mine && c < 2) out[2 * r] = Ln;
+    L = c < 2 ? dn : nb;
+  }
+  if (mine && c < 2) col[2 * nt] = L;
+  return ok;
+}
+
 // A subdiagonal below one unit of roundoff of its neighbours' diagonal deflates if the refined test
 // agrees (Ahues and Tisseur). Where both diagonal entries are the same number (equal eigenvalues of a
 // uniform layer, split by rounding alone) that test never does, and when the shift rounds to them too
@@ -886,7 +1109,9 @@ __global__ void __launch_bounds__(QrMaxThreads<R>::v) hseqr_kernel(Cx<R>* __rest
   // Warps of the chasing CTA: 0 chases, 1 follows with the near columns, 0 .. 3 bring in a sweep's
   // first tile. Its far updates keep off the chasing warp's scheduler (every fourth warp); in the
   // 16-byte forms of a cluster the CTA leaves them to the others.
-  const bool chaser = rank == 0 && warp == 0, near = rank == 0 && warp == 1, helper = rank == 0 && warp < 4;
+  constexpr bool f64 = std::is_same<R, double>::value;
+  const bool chaser = rank == 0 && warp == 0, near = rank == 0 && warp >= 1 && warp <= (f64 ? 2 : 1);
+  const bool helper = rank == 0 && warp < 4;
   int worker = -1, nworkers;                                 // CTA by CTA within each round of tasks
   {
     const int nw = blockDim.x >> 5, own = (sizeof(R) > 4 && ctas > 1) ? 0 : nw - (nw + 3) / 4 - 1, c = (int)ctas;
@@ -917,13 +1142,19 @@ __global__ void __launch_bounds__(QrMaxThreads<R>::v) hseqr_kernel(Cx<R>* __rest
       }
     }
     if (near && s_req.k0 >= 0 && s_req.k1 < s_req.i) {
-      const bool ok = qr::near_columns<R>(H, ldh, tile + (s_req.tile ^ 1) * TS, s_req, rec[buf], rec[prev], s_bar,
-                                          followed & 1u);
+      bool ok;
+      if constexpr (f64)
+        ok = qr::near_columns64(H, ldh, tile + (s_req.tile ^ 1) * TS, s_req, warp - 1, rec[buf], rec[prev], s_bar, followed & 1u);
+      else
+        ok = qr::near_columns<R>(H, ldh, tile + (s_req.tile ^ 1) * TS, s_req, rec[buf], rec[prev], s_bar, followed & 1u);
       ++followed;
       if (!ok) s_late = 1;
     }
     if (chaser) {
-      if (type == kQrWindow) qr::chase_window<R>(H, ldh, tile + s_req.tile * TS, s_req, cs, rec[buf], s_bar);
+      if (type == kQrWindow) {
+        if constexpr (f64) qr::chase_window64(H, ldh, tile + s_req.tile * TS, s_req, cs, rec[buf], s_bar);
+        else qr::chase_window<R>(H, ldh, tile + s_req.tile * TS, s_req, cs, rec[buf], s_bar);
+      }
       rec[buf].type = type;
       __syncwarp();
       if (ctas > 1) qr::send_record<R>(rec[buf], ctas);
