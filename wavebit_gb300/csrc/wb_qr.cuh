@@ -181,6 +181,45 @@ __device__ __forceinline__ Cx<float> wilkinson(Cx<float> p, Cx<float> u1, Cx<flo
   }
   return left_sub(t, u, q);
 }
+// 1 / sqrt(v) to 22 bits for normal v > 0, from the FP32 unit; the exponents by integer operations
+// (a conversion costs as much as an FP64 operation).
+__device__ __forceinline__ double rsqrt_start(double v) {
+  int hi = __double2hiint(v);
+  const int k = ((hi >> 20) - 1023) & ~1;
+  hi -= k * (1 << 20);                                          // v / 2^k in [1, 4)
+  float f = __int_as_float((int)(((unsigned)(hi - (896 << 20)) << 3) | ((unsigned)__double2loint(v) >> 29)));
+  asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(f));
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double((int)(b >> 3) + (896 - (k >> 1)) * (1 << 20), (int)(b << 29));
+}
+
+// 1 / sqrt(v): one third-order step from there (the error's cube times 5/16 is below 2^-64)
+__device__ __forceinline__ double rsqrt64(double v) {
+  const double y = rsqrt_start(v), d = fma(-(v * y), y, 1.0);
+  return fma(y, d * fma(d, 0.375, 0.5), y);
+}
+// The same eigenvalue in FP64: t - u1 u2 / (x + y), y^2 = x^2 + u1 u2, x = (p - t) / 2. In FP64 a division
+// or a root costs 7 to 10 multiply-adds of 64 cycles; these are three of the reciprocal roots above. Entries
+// out of 2^+-200 go the scaled way.
+__device__ __forceinline__ Cx<double> wilkinson(Cx<double> p, Cx<double> u1, Cx<double> u2, Cx<double> t) {
+  auto hi = [](double v) { return __double2hiint(v) & 0x7fffffff; };
+  const Cx<double> x = (p - t) * 0.5;
+  const int e = max(max(hi(x.x), hi(x.y)), max(max(hi(u1.x), hi(u1.y)), max(hi(u2.x), hi(u2.y)))) >> 20;
+  if ((unsigned)(e - (1023 - 200)) > 400u) return wilkinson<double>(p, u1, u2, t);
+  const Cx<double> w = u1 * u2, z = x * x + w;
+  Cx<double> y = cxzero<double>();
+  if (max(hi(z.x), hi(z.y)) >> 20 > 1023 - 500) {               // principal root of z
+    const double m2 = fma(z.x, z.x, z.y * z.y), t2 = 0.5 * fma(m2, rsqrt64(m2), fabs(z.x));
+    const double rt = rsqrt64(t2), a = t2 * rt, b = 0.5 * (z.y * rt);
+    y = z.x >= 0.0 ? cxmk<double>(a, b) : cxmk<double>(fabs(b), z.y < 0.0 ? -a : a);
+  }
+  if (fma(x.x, y.x, x.y * y.y) < 0.0) y = -y;
+  const Cx<double> d = x + y;
+  const double dd = fma(d.x, d.x, d.y * d.y);
+  if (hi(dd) >> 20 < 1023 - 900) return t;                      // x = 0 = u1 u2
+  const double r = rsqrt64(dd);
+  return t - w * cxconj(d) * (r * r);
+}
 }  // namespace qr
 
 // Reflector of (alpha, x) with x real, as used by the chase: beta = -sign(Re alpha)|(alpha, x)|,
@@ -684,105 +723,85 @@ __device__ __forceinline__ double flip(double v, int mask) {    // v with its si
 }
 __device__ __forceinline__ double shx(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
 
-// 1 / sqrt(v) to 22 bits for normal v > 0, from the FP32 unit; the exponents by integer operations
-// (a conversion costs as much as an FP64 operation).
-__device__ __forceinline__ double rsqrt_start(double v) {
-  int hi = __double2hiint(v);
-  const int k = ((hi >> 20) - 1023) & ~1;
-  hi -= k * (1 << 20);                                          // v / 2^k in [1, 4)
-  float f = __int_as_float((int)(((unsigned)(hi - (896 << 20)) << 3) | ((unsigned)__double2loint(v) >> 29)));
-  asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(f));
-  const unsigned b = __float_as_uint(f);
-  return __hiloint2double((int)(b >> 3) + (896 - (k >> 1)) * (1 << 20), (int)(b << 29));
-}
-
 struct Chase64 {
   double L[3];                 // left layout: this lane's component of its pair in every set
-  double eu, ev, ew;           // right layout, rows k - 1 and k + 2: the component and its partners
+  double e;                    // right layout: rows k - 1 and k + 2
   double cx, cy, s;            // the rotation
+  const double* in;            // left layout, set 0: row k + 2 of column k + 1 + slot (the next step's) in the tile
+  const double* sub;           // (k + 3, k + 2) in the tile
+  double* out;                 // row k of column k + slot in H
+  double* band;                // right layout: row k - 1 + slot of column k + c / 2 in H
+  double* rec;                 // lanes 0 .. 2: the rotation's parts in the record
 };
 
 template <int NS>
-__device__ __forceinline__ void chase64_step(Chase64& v, Cx<double>* H, int ldh, const double* tile, int q, int k0, int o,
-                                             int i, int cmax, bool lastw, QrRecord<double>& g, uint64_t* bars) {
-  constexpr int MW = QrWin<double>::m, TL = QrTile<double>::ld;
-  const int lane = threadIdx.x & 31, c = lane & 3, slot = lane >> 2, k = k0 + q;
+__device__ __forceinline__ void chase64_step(Chase64& v, Cx<double>* H, int ldh, int k, int i, int cmax,
+                                             QrRecord<double>& g) {
+  constexpr int TL = QrTile<double>::ld;
+  const int lane = threadIdx.x & 31, c = lane & 3, slot = lane >> 2;
   const int left = (c == 1 || c == 2) ? 1 << 31 : 0, rest = c >= 2 ? 1 << 31 : 0;
-  const int col2 = (c >> 1) * 4 + (c & 1);                      // row k of column k + c / 2
-  if (lane < 2) reinterpret_cast<double*>(&g.t1[q])[lane] = lane ? v.cy : v.cx;
-  if (lane == 2) g.t2[q] = v.s;
-  // the rows the next step needs: row k + 2 of the columns, (k + 3, k + 2)
-  double nb[NS];
-#pragma unroll
-  for (int t = 0; t < NS; ++t) {
-    const int jj = q - 1 + 8 * t + slot;
-    const bool in = jj >= 0 && jj < MW && k0 + 2 + jj <= cmax;
-    nb[t] = in ? tile[2 * (jj * TL + o + q + 2) + (c & 1)] : 0.0;
-  }
-  const double n21x = tile[2 * (q * TL + o + q + 3)], n21y = tile[2 * (q * TL + o + q + 3) + 1];
+  const int col2 = ((c >> 1) * 4 + (c & 1)) | (lane & 8 ? 2 : 0);   // slot 1: row k, slot 2: row k + 1 of column k + c / 2
   // left on columns k ..
   const double cyl = flip(v.cy, left), sl = flip(v.s, rest);
-  double Ln[NS];
-#pragma unroll
-  for (int t = 0; t < NS; ++t) Ln[t] = fma(v.cx, v.L[t], fma(cyl, shx(v.L[t], 1), sl * shx(v.L[t], 2)));
+  double Ln[NS], nb[NS];
+  Ln[0] = fma(v.cx, v.L[0], fma(cyl, shx(v.L[0], 1), sl * shx(v.L[0], 2)));
+  if (lane < 3) *v.rec = lane == 0 ? v.cx : lane == 1 ? v.cy : v.s;
   // right on rows k - 1 .. k + 2 of columns k, k + 1; lane 16 makes the square of (k + 2, k)
-  double u = shf(Ln[0], (lane & 8 ? 2 : 0) + col2), pv = shf(Ln[0], ((lane & 8 ? 2 : 0) + col2) ^ 1);
-  double pw = shf(Ln[0], ((lane & 8 ? 2 : 0) + col2) ^ 4);
-  if (slot != 1 && slot != 2) { u = v.eu; pv = v.ev; pw = v.ew; }
+  const double ev = shx(v.e, 1), ew = shx(v.e, 2);
+  double u = shf(Ln[0], col2), pv = shf(Ln[0], col2 ^ 1), pw = shf(Ln[0], col2 ^ 4);
+  if (slot != 1 && slot != 2) { u = v.e; pv = ev; pw = ew; }
   const double r1 = sl * pw;
   const bool sq = slot == 4;
   const double r2 = fma(sq ? r1 : flip(cyl, 1 << 31), sq ? r1 : pv, sq ? 0.0 : r1);
   const double Rn = fma(v.cx, u, r2);
-  const double ax = shf(Rn, 8), ay = shf(Rn, 9), xx = shf(Rn, 12), x2 = shf(Rn, 16);
-  // the finished row k of the columns past k + 2
+  // the rows the next step needs: row k + 2 of its columns, (k + 3, k + 2). A column past the window's
+  // reads what the tile happens to hold there: it never joins the core.
 #pragma unroll
-  for (int t = 0; t < NS; ++t) {
-    const int col = k + 8 * t + slot;
-    if (c < 2 && 8 * t + slot >= 3 && col <= cmax) reinterpret_cast<double*>(H + k + (long long)col * ldh)[c] = Ln[t];
-  }
-  double subx = ax, suby = ay;
+  for (int t = 0; t < NS; ++t) nb[t] = v.in[t == 0 && slot == 0 ? 2 * TL : 16 * t * TL];
+  const double n21 = v.sub[c & 1];
+#pragma unroll
+  for (int t = 1; t < NS; ++t) Ln[t] = fma(v.cx, v.L[t], fma(cyl, shx(v.L[t], 1), sl * shx(v.L[t], 2)));
+  const double ax = shf(Rn, 8), ay = shf(Rn, 9), xx = shf(Rn, 12), x2 = shf(Rn, 16);
   double top = Rn;                                              // what the band keeps, right layout
   if (k + 1 < i) {
     const int e = max(max(__double2hiint(ax) & 0x7fffffff, __double2hiint(ay) & 0x7fffffff), __double2hiint(xx) & 0x7fffffff) >> 20;
-    if (e < 1023 - 400 || e > 1023 + 400 || (xx == 0.0 && ay == 0.0)) {
+    double beta, z0 = 0.0;
+    if ((unsigned)(e - (1023 - 400)) > 800u) {
       const Rot<double> rn = chase_reflector<double>(cxmk<double>(ax, ay), xx);
-      if (!rn.identity) { subx = rn.beta; suby = 0.0; }
+      beta = rn.beta;
+      if (rn.identity) z0 = ay;
       v.cx = rn.t1.x; v.cy = rn.t1.y; v.s = rn.t2;
     } else {
       // (ax, ay, xx, ss) / sqrt(ss), one a lane, by one third-order step from a 22-bit start
       const double ss = fma(ax, ax, fma(ay, ay, x2)), y = rsqrt_start(ss);
       const double z = (c == 0 ? ax : c == 1 ? ay : c == 2 ? xx : ss) * y;
       const double d = fma(-shf(z, 3), y, 1.0);
-      const double res = fma(z, d * fma(d, 0.375, 0.5), z);
-      v.cx = shf(res, 0); v.cy = shf(res, 1); v.s = shf(res, 2);
-      subx = shf(res, 3); suby = 0.0;
+      beta = fma(z, d * fma(d, 0.375, 0.5), z);
+      v.cx = shf(beta, 0); v.cy = shf(beta, 1); v.s = shf(beta, 2);   // c == 3 keeps sqrt(ss)
     }
     // the pairs of step k + 1
     double m[NS];
 #pragma unroll
     for (int t = 0; t < NS; ++t) m[t] = shf(Ln[t], (lane + 6) & 31);
     const double core = shf(Rn, 10 + (c & 1) + 4 * (c >> 1));
+    const double xy = shf(slot == 1 ? Rn : Ln[0], 6 + c);       // (k, k + 1), (k, k + 2)
 #pragma unroll
     for (int t = 0; t < NS; ++t) v.L[t] = c >= 2 ? nb[t] : slot < 7 ? m[t] : t + 1 < NS ? m[t + 1 < NS ? t + 1 : t] : 0.0;
     if (slot == 0) v.L[0] = core;
-    const double xn = shf(Rn, 6 + (c & 1)), yn = shf(Ln[0], 8 + (c & 1));
-    const double xo = shx(xn, 1), yo = shx(yn, 1);
-    v.eu = slot == 0 ? (c < 2 ? xn : yn) : 0.0;
-    v.ev = slot == 0 ? (c < 2 ? xo : yo) : 0.0;
-    v.ew = slot == 0 ? (c < 2 ? yn : xn) : c == 0 ? n21x : c == 1 ? n21y : 0.0;
-    if (slot == 3 && c >= 2) { v.eu = c == 2 ? n21x : n21y; v.ev = c == 2 ? n21y : n21x; }
+    v.e = slot == 0 ? xy : c >= 2 ? n21 : 0.0;
+    if (slot < 2 && (slot == 0 || c < 2) && (slot > 0 || k > 0)) *v.band = top;
+    if (slot == 2 && c >= 2) v.band[c == 3 ? -1 : 0] = c == 3 ? beta : z0;
   } else {
     // the sweep's last subdiagonal made real; the factor goes to column k + 1
     Cx<double> sc = cxone<double>();
+    double subx = ax;
     int scaled = 0;
     if (ay != 0.0) {
       const double am = modulus(cxmk<double>(ax, ay));
       if (am > RealT<double>::tiny()) {
-        subx = am; suby = 0.0;
+        subx = am;
         sc = cxmk<double>(ax, ay) * (1.0 / am);
         scaled = 1;
-      } else {
-        suby = 0.0;
       }
     }
     const double other = shx(Rn, 1);
@@ -792,13 +811,19 @@ __device__ __forceinline__ void chase64_step(Chase64& v, Cx<double>* H, int ldh,
       top = c == 2 ? w.x : w.y;
     }
     if (lane == 0) { g.sc = sc; g.scaled = scaled; }
-    if (c >= 2 && (slot == 1 || slot == 2)) reinterpret_cast<double*>(H + (i - 2 + slot) + (long long)i * ldh)[c - 2] = top;
+    if (slot == 2 && c < 2) top = c ? 0.0 : subx;
+    double* at = slot == 2 && c >= 2 ? v.band + 2 * ldh - 3 + c : v.band;
+    if (slot < 3 && (slot > 0 || k > 0)) *at = top;             // rows k, k + 1 of column k + 1 too
   }
-  if (slot == 2 && c < 2) top = c ? suby : subx;
-  if (slot < 3 && (slot == 0 || c < 2) && (slot > 0 || k > 0))
-    reinterpret_cast<double*>(H + (k - 1 + slot) + (long long)(k + (c >> 1)) * ldh)[c & 1] = top;
-  __syncwarp();
-  if (!lastw && (q + 1) % kQrStride == 0 && lane == 0) publish(bars, q / kQrStride);
+  // the finished row k of the columns past k + 2
+#pragma unroll
+  for (int t = 0; t < NS; ++t)
+    if (c < 2 && 8 * t + slot >= 3 && k + 8 * t + slot <= cmax) v.out[16LL * t * ldh] = Ln[t];
+  v.in += 2 * (TL + 1);
+  v.sub += 2 * (TL + 1);
+  v.out += 2 * (ldh + 1);
+  v.band += 2 * (ldh + 1);
+  v.rec += lane < 2 ? 2 : 1;
 }
 
 __device__ __noinline__ void chase_window64(Cx<double>* H, int ldh, const Cx<double>* tile, const Request& rq,
@@ -819,31 +844,35 @@ __device__ __noinline__ void chase_window64(Cx<double>* H, int ldh, const Cx<dou
   auto part = [](const Cx<double>& a, int p) { return p ? a.y : a.x; };
   if (slot == 0) v.L[0] = part(c < 2 ? cs.c00 : cs.c10, c & 1);
   if (slot == 1) v.L[0] = part(c < 2 ? cs.c01 : cs.c11, c & 1);
-  v.eu = v.ev = v.ew = 0.0;
-  if (slot == 0) {
-    v.eu = part(c < 2 ? cs.x : cs.y, c & 1);
-    v.ev = part(c < 2 ? cs.x : cs.y, (c & 1) ^ 1);
-    v.ew = part(c < 2 ? cs.y : cs.x, c & 1);
-  } else if (c < 2) {
-    v.ew = part(cs.c21, c);
-  } else if (slot == 3) {
-    v.eu = part(cs.c21, c & 1);
-    v.ev = part(cs.c21, (c & 1) ^ 1);
-  }
+  v.e = slot == 0 ? part(c < 2 ? cs.x : cs.y, c & 1) : c >= 2 ? part(cs.c21, c & 1) : 0.0;
   v.cx = cs.t1.x; v.cy = cs.t1.y; v.s = cs.t2;
+  v.in = td + 2 * ((slot - 1) * TL + o + 2) + (c & 1);         // the core's column (slot 0, set 0) reads the next one's
+  v.sub = td + 2 * (o + 3);
+  v.out = reinterpret_cast<double*>(H + k0 + (long long)(k0 + slot) * ldh) + (c & 1);
+  v.band = reinterpret_cast<double*>(H + (k0 - 1 + slot) + (long long)(k0 + (c >> 1)) * ldh) + (c & 1);
+  if (slot == 2 && c >= 2) v.band = reinterpret_cast<double*>(H + k0 + 1 + (long long)k0 * ldh) + 1;
+  v.rec = lane < 2 ? reinterpret_cast<double*>(g.t1) + lane : g.t2;
   __syncwarp();
   if (lane == 0) { g.sc = cxone<double>(); g.scaled = 0; }
   const int nc = cmax - k0 + 1;                                 // columns at the window's first step
   int q = 0;
+  auto done = [&]() {
+    ++q;
+    if (q % kQrStride == 0) {
+      __syncwarp();
+      if (!lastw && lane == 0) publish(bars, q / kQrStride - 1);
+    }
+  };
 #pragma unroll 1
-  for (; q < k1 - k0 && nc - q > 16; ++q) chase64_step<3>(v, H, ldh, td, q, k0, o, i, cmax, lastw, g, bars);
+  while (q < k1 - k0 && nc - q > 16) { chase64_step<3>(v, H, ldh, k0 + q, i, cmax, g); done(); }
 #pragma unroll 1
-  for (; q < k1 - k0 && nc - q > 8; ++q) chase64_step<2>(v, H, ldh, td, q, k0, o, i, cmax, lastw, g, bars);
+  while (q < k1 - k0 && nc - q > 8) { chase64_step<2>(v, H, ldh, k0 + q, i, cmax, g); done(); }
 #pragma unroll 1
-  for (; q < k1 - k0; ++q) chase64_step<1>(v, H, ldh, td, q, k0, o, i, cmax, lastw, g, bars);
+  while (q < k1 - k0) { chase64_step<1>(v, H, ldh, k0 + q, i, cmax, g); done(); }
+  __syncwarp();
   if (slot < 2) reinterpret_cast<double*>(slot ? (c < 2 ? &cs.c01 : &cs.c11) : (c < 2 ? &cs.c00 : &cs.c10))[c & 1] = v.L[0];
-  if (slot == 0) reinterpret_cast<double*>(c < 2 ? &cs.x : &cs.y)[c & 1] = v.eu;
-  if (slot == 3 && c >= 2) reinterpret_cast<double*>(&cs.c21)[c & 1] = v.eu;
+  if (slot == 0) reinterpret_cast<double*>(c < 2 ? &cs.x : &cs.y)[c & 1] = v.e;
+  if (slot == 3 && c >= 2) reinterpret_cast<double*>(&cs.c21)[c & 1] = v.e;
   if (lane == 0) {
     const int k2 = min(k1 + MW, i), k3 = min(k2 + MW, i);
     g.k0 = k0; g.k1 = k1;
@@ -922,7 +951,29 @@ __device__ __noinline__ int next_window(Cx<R>* H, int n, int ldh, Cx<R>* w, int 
       if (i < 0) { type = kQrDone; break; }
       // largest k in [1, i] with a negligible subdiagonal H(k, k-1), 0 when there is none
       int cand = 0;
+      unsigned maybe = ~0u;                                // chunks of 32 of the next 128 that have to be looked at
       for (int kb = i; kb >= 1; kb -= 32) {
+        if constexpr (std::is_same<R, double>::value) {
+          // By the exponents alone (integers): |sub| > 2^-49 of the largest part of its neighbours stays.
+          if (((i - kb) & 96) == 0) {
+            bool any[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int k = kb - 32 * u - lane;
+              any[u] = false;
+              if (k >= 1) {
+                const C_ hd = hl(k, k), hp = hl(k - 1, k - 1);
+                auto hi = [](double v) { return __double2hiint(v) & 0x7fffffff; };
+                const int es = hi(hl(k, k - 1).x) >> 20, em = max(max(hi(hd.x), hi(hd.y)), max(hi(hp.x), hi(hp.y))) >> 20;
+                any[u] = es <= max(em - 48, 100) || em == 0;
+              }
+            }
+            maybe = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) maybe |= __any_sync(0xffffffffu, any[u]) ? 1u << u : 0u;
+          }
+          if (!(maybe >> (((i - kb) >> 5) & 3) & 1u)) continue;
+        }
         const int k = kb - lane;
         bool small = false;
         if (k >= 1) {
@@ -982,7 +1033,9 @@ __device__ __noinline__ int next_window(Cx<R>* H, int n, int ldh, Cx<R>* w, int 
       if (sc == R(0.0)) sc = R(1.0);
       R isc = R(1.0) / sc;
       // the first reflector of the sweep, from the shifted first column
-      Rot<R> rf = chase_reflector(h11s * isc, h21 * isc);
+      Rot<R> rf;
+      if constexpr (std::is_same<R, double>::value) rf = chase_reflector<R>(h11s, h21);   // scales by itself
+      else rf = chase_reflector(h11s * isc, h21 * isc);
       k0 = l;
       __syncwarp();
       if (lane == 0) {
