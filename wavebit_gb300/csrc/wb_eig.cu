@@ -97,6 +97,9 @@ template <class R> __device__ __forceinline__ Refl<R> make_reflector(Cx<R> alpha
   return r;
 }
 
+}  // namespace wb
+#include "wb_hrd.cuh"
+namespace wb {
 // ------------------------------------------------------------- 1. Hessenberg reduction
 // H := Q^H A Q, reflectors stored below the subdiagonal (v_0 = 1 implicit), tau[k].
 //
@@ -898,6 +901,49 @@ int hrd_threads(int batch, int n) {
   return t;
 }
 
+// Launches kernel with `ctas` CTAs a matrix as one cluster.
+template <class... P, class... Q>
+static void launch_cluster(cudaStream_t s, void (*kernel)(P...), int ctas, int batch, int threads, size_t smem, Q... args) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(batch * ctas));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)ctas;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  note_launch();
+}
+
+// FP64, n > kQrSmall: H and Q by wb_hrd.cuh; false where its shared memory does not reach.
+static bool reduce64(cudaStream_t s, int batch, int n, Cx<double>* A, int lda, long long a_bs, Cx<double>* Z, int ldz,
+                     long long z_bs, Cx<double>* tau) {
+  const size_t smem = hrd::shared_elements(n) * sizeof(Cx<double>);
+  if (n > 512 || smem > 200 * 1024) return false;
+  const int sms = sm_count();
+  int c = 1;
+  while (2 * c <= hrd::kParts && 2LL * c * batch <= sms) c *= 2;
+  if (n <= 64) launch_cluster(s, hrd::gehrd64_kernel<2>, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
+  else if (n <= 128) launch_cluster(s, hrd::gehrd64_kernel<4>, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
+  else launch_cluster(s, hrd::gehrd64_kernel<8>, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
+  const int groups = n <= 256 ? (n + 1) / 2 : n;
+  const unsigned gx = (unsigned)max(1LL, min((long long)(groups + 3) / 4, (2LL * sms + batch - 1) / batch));
+  const dim3 grid(gx, (unsigned)batch);
+  if (n <= 64) hrd::unghr64_kernel<2, 2><<<grid, 128, 0, s>>>(A, n, lda, a_bs, tau, Z, ldz, z_bs);
+  else if (n <= 128) hrd::unghr64_kernel<4, 2><<<grid, 128, 0, s>>>(A, n, lda, a_bs, tau, Z, ldz, z_bs);
+  else if (n <= 256) hrd::unghr64_kernel<8, 2><<<grid, 128, 0, s>>>(A, n, lda, a_bs, tau, Z, ldz, z_bs);
+  else hrd::unghr64_kernel<16, 1><<<grid, 128, 0, s>>>(A, n, lda, a_bs, tau, Z, ldz, z_bs);
+  note_launch();
+  const unsigned cx = (unsigned)min((long long)sms, ((long long)n * n + 255) / 256);
+  clear_below_subdiag_kernel<double><<<dim3(cx, (unsigned)batch), 256, 0, s>>>(A, n, lda, a_bs); note_launch();
+  return true;
+}
+
 template <class R>
 void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a_bs, Cx<R>* Z, int ldz,
                 long long z_bs, Cx<R>* w, Cx<R>* tau, int32_t* status, int st_div, Cx<R>* ws, long long ws_bs,
@@ -910,7 +956,12 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
   // the FP32 form at n >= 192 reduces in panels (Z, not yet formed, holds the panels' scratch:
   // 5 n kHrdPanel + kHrdPanel^2 elements, within n * ldz from n = 161 on)
   const bool blocked = sizeof(R) == 4 && n >= 192 && ldz >= n && tuning(kTuneHrdBlocked) != 1;
-  if (blocked) {
+  bool reduced = false;
+  if constexpr (std::is_same<R, double>::value) {
+    if (n > kQrSmall) reduced = reduce64(s, batch, n, A, lda, a_bs, Z, ldz, z_bs, tau);
+  }
+  if (reduced) {
+  } else if (blocked) {
     cudaFuncSetAttribute(gehrd_panel_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     const int BB = kHrdPanel;
     const long long nB = (long long)n * BB;
@@ -938,7 +989,8 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
     gehrd_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, live); note_launch();
   }
   // Q in panels when the caller lends scratch (5 n kHrdPanel + kHrdPanel^2 elements a matrix)
-  if (blocked && ws && ws_bs >= 5LL * n * kHrdPanel + kHrdPanel * kHrdPanel) {
+  if (reduced) {
+  } else if (blocked && ws && ws_bs >= 5LL * n * kHrdPanel + kHrdPanel * kHrdPanel) {
     const int BB = kHrdPanel;
     const long long nB = (long long)n * BB;
     Cx<R>* V = ws;
@@ -965,18 +1017,6 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
   }
   int itmax = 30 * (n > 10 ? n : 10);
   const QrShape shape = qr_shape<R>(batch, n);
-  cudaFuncSetAttribute(hseqr_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(batch * shape.ctas));
-  cfg.blockDim = dim3((unsigned)shape.threads);
-  cfg.dynamicSmemBytes = shape.smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)shape.ctas;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   bool timed = false;
   {
@@ -995,9 +1035,10 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
       launched = true;
     }
   }
-  if (!launched)
-    cudaLaunchKernelEx(&cfg, hseqr_kernel<R>, A, n, lda, a_bs, Z, ldz, z_bs, w, status, st_div < 1 ? 1 : st_div, itmax);
-  note_launch();
+  if (launched) note_launch();
+  else
+    launch_cluster(s, hseqr_kernel<R>, shape.ctas, batch, shape.threads, shape.smem, A, n, lda, a_bs, Z, ldz, z_bs, w,
+                   status, st_div < 1 ? 1 : st_div, itmax);
   if (timed) cudaEventRecord(e1, s);
 }
 
