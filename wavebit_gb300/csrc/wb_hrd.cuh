@@ -68,14 +68,14 @@ __device__ __forceinline__ Refl<double> reflector(C64 alpha, double xn2) {
   const double ss = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn2));
   if ((unsigned)((hi(ss) >> 20) - (1023 - 400)) > 800u || xn2 == 0.0) return make_reflector<double>(alpha, sqrt(xn2));
   Refl<double> r;
-  const double rs = qr::rsqrt64(ss), nrm = ss * rs;
+  const double rs = rsqrt64(ss), nrm = ss * rs;
   const bool neg = alpha.x < 0.0;
   r.identity = false;
   r.beta = neg ? nrm : -nrm;
   const double ib = neg ? rs : -rs;
   r.tau = cxmk<double>(fma(-alpha.x, ib, 1.0), -alpha.y * ib);
   const C64 d = cxmk<double>(alpha.x - r.beta, alpha.y);
-  const double rd = qr::rsqrt64(fma(d.x, d.x, d.y * d.y)), ir = rd * rd;
+  const double rd = rsqrt64(fma(d.x, d.x, d.y * d.y)), ir = rd * rd;
   r.scale = cxmk<double>(d.x * ir, -d.y * ir);
   return r;
 }

@@ -787,8 +787,22 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
     note_launch();
   }
   const size_t sm = sizeof(Cx<R>) * (size_t)TB_NB * (TB_NB + 1);
-  cudaFuncSetAttribute(tri::trsm_diag_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  const dim3 gd((nrhs + tri::kTriThreads / 8 - 1) / (tri::kTriThreads / 8), batch);
+  // threads a column: FP32 is bound by the block's chain of shuffles; FP64 by the instructions of a warp
+  // times the warps a scheduler gets
+  int T = 8;
+  auto kernel = tri::trsm_diag_kernel<R, 8>;
+  if constexpr (std::is_same<R, double>::value) {
+    long long least = 1LL << 62;
+    for (int t = 8, cost = 1152; t <= 32; t *= 2, cost = t == 16 ? 640 : 384) {
+      const long long warps = (nrhs + 32 / t - 1) / (32 / t) * (long long)batch, per = 4LL * sm_count();
+      const long long rounds = (warps + per - 1) / per;
+      if (rounds * cost < least) { least = rounds * cost; T = t; }
+    }
+    if (T == 16) kernel = tri::trsm_diag_kernel<R, 16>;
+    if (T == 32) kernel = tri::trsm_diag_kernel<R, 32>;
+  }
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const dim3 gd((nrhs + tri::kTriThreads / T - 1) / (tri::kTriThreads / T), batch);
   auto diagonal = [&](int i0, int ib, int lower, int unit) {
     if constexpr (sizeof(R) == 4) {
       if (!lower) {
@@ -800,7 +814,7 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
         return;
       }
     }
-    tri::trsm_diag_kernel<R><<<gd, tri::kTriThreads, sm, s>>>(LU, lda, a_bs, B, nrhs, ldb, b_bs, i0, ib, lower, unit, trans);
+    kernel<<<gd, tri::kTriThreads, sm, s>>>(LU, lda, a_bs, B, nrhs, ldb, b_bs, i0, ib, lower, unit, trans);
     note_launch();
   };
   const double2 m1 = make_double2(-1.0, 0.0), p1 = make_double2(1.0, 0.0);
@@ -844,8 +858,8 @@ void getrs(cudaStream_t s, int batch, int n, const Cx<R>* LU, int lda, long long
     return;
   }
   constexpr bool fp64 = std::is_same<R, double>::value;
-  if constexpr (fp64) {          // FP64: from 8 columns on (n = 50: 580 -> 110 us)
-    if (nrhs >= 8) {
+  if constexpr (fp64) {          // FP64: from 8 columns on (n = 50: 580 -> 110 us); transposed, any number
+    if (nrhs >= 8 || (trans && n > 16)) {
       getrs_blocked<R>(s, batch, n, LU, lda, a_bs, ipiv, piv_bs, B, nrhs, ldb, b_bs, trans);
       return;
     }

@@ -181,23 +181,6 @@ __device__ __forceinline__ Cx<float> wilkinson(Cx<float> p, Cx<float> u1, Cx<flo
   }
   return left_sub(t, u, q);
 }
-// 1 / sqrt(v) to 22 bits for normal v > 0, from the FP32 unit; the exponents by integer operations
-// (a conversion costs as much as an FP64 operation).
-__device__ __forceinline__ double rsqrt_start(double v) {
-  int hi = __double2hiint(v);
-  const int k = ((hi >> 20) - 1023) & ~1;
-  hi -= k * (1 << 20);                                          // v / 2^k in [1, 4)
-  float f = __int_as_float((int)(((unsigned)(hi - (896 << 20)) << 3) | ((unsigned)__double2loint(v) >> 29)));
-  asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(f));
-  const unsigned b = __float_as_uint(f);
-  return __hiloint2double((int)(b >> 3) + (896 - (k >> 1)) * (1 << 20), (int)(b << 29));
-}
-
-// 1 / sqrt(v): one third-order step from there (the error's cube times 5/16 is below 2^-64)
-__device__ __forceinline__ double rsqrt64(double v) {
-  const double y = rsqrt_start(v), d = fma(-(v * y), y, 1.0);
-  return fma(y, d * fma(d, 0.375, 0.5), y);
-}
 // The same eigenvalue in FP64: t - u1 u2 / (x + y), y^2 = x^2 + u1 u2, x = (p - t) / 2. In FP64 a division
 // or a root costs 7 to 10 multiply-adds of 64 cycles; these are three of the reciprocal roots above. Entries
 // out of 2^+-200 go the scaled way.

@@ -52,18 +52,74 @@ constexpr int kUpdate = 2, kScale = 0;
 
 // ------------------------------------------------------------------------------------ LU panel
 // Partial pivoting down a panel of kPB columns, by a cluster of C CTAs a matrix: the panel's rows in the
-// CTAs' shared memory (column by column, `rows` each), kSlices threads a row. Per column: the largest
-// |re| + |im| (first index on ties) over the cluster, the pivot row and row j exchanged and broadcast,
-// then every row's multiplier and update.
+// CTAs' shared memory (column by column, `rows` each), `slices` threads a row. Per column: every CTA sends
+// its largest |re| + |im| (first index on ties) with that row to the others, the owner of row j its row,
+// and after one cluster barrier each picks the pivot, exchanges its rows, scales its multipliers and
+// updates; the threads that update column j + 1 start its search. What they receive is buffered twice,
+// so the next column's barrier is the only one.
+//
+// The magnitudes are compared as integers (an FP64 compare holds a scheduler for 64 cycles, as any FP64
+// instruction; the search and its exchange took half of a column's 13000 cycles with them).
 constexpr int kPB = 32;
 constexpr int kPanelThreads = 512;
 constexpr int kPanelMaxCluster = 8;
 
+// Magnitudes in order: non-negative values' bits are; NaN and nothing below them all.
+template <class R> struct Mag {
+  R v;
+  static __device__ __forceinline__ Mag none() { Mag m; m.v = R(-1.0); return m; }
+  static __device__ __forceinline__ Mag of(R a) { Mag m; m.v = a >= R(0.0) ? a : R(-1.0); return m; }
+  __device__ __forceinline__ bool operator>(const Mag& o) const { return v > o.v; }
+  __device__ __forceinline__ bool operator==(const Mag& o) const { return v == o.v; }
+  __device__ __forceinline__ Mag lane(int src) const { Mag m; m.v = shf(v, src); return m; }
+};
+template <> struct Mag<float> {
+  int v;
+  static __device__ __forceinline__ Mag none() { return {-1}; }
+  static __device__ __forceinline__ Mag of(float a) { const int b = __float_as_int(a); return {b > 0x7f800000 ? -1 : b}; }
+  __device__ __forceinline__ bool operator>(const Mag& o) const { return v > o.v; }
+  __device__ __forceinline__ bool operator==(const Mag& o) const { return v == o.v; }
+  __device__ __forceinline__ Mag lane(int src) const { return {__shfl_sync(0xffffffffu, v, src)}; }
+};
+template <> struct Mag<double> {
+  long long v;
+  static __device__ __forceinline__ Mag none() { return {-1}; }
+  static __device__ __forceinline__ Mag of(double a) {
+    const long long b = __double_as_longlong(a);
+    return {b > 0x7ff0000000000000ll ? -1 : b};
+  }
+  __device__ __forceinline__ bool operator>(const Mag& o) const { return v > o.v; }
+  __device__ __forceinline__ bool operator==(const Mag& o) const { return v == o.v; }
+  __device__ __forceinline__ Mag lane(int src) const { return {__shfl_sync(0xffffffffu, v, src)}; }
+};
+template <class R> struct Pivot {
+  Mag<R> m;
+  int i;
+  __device__ __forceinline__ void take(const Mag<R>& om, int oi) {
+    if (om > m || (om == m && oi < i)) { m = om; i = oi; }
+  }
+  __device__ __forceinline__ void meet(int o, int lane) {
+    const Mag<R> om = m.lane(lane ^ o);
+    take(om, __shfl_xor_sync(0xffffffffu, i, o));
+  }
+};
+
+// 1 / p: in FP64 conj(p) / |p|^2 by one reciprocal root (Smith's three divisions cost 1400 cycles of a
+// column's chain)
+template <class R> __device__ __forceinline__ Cx<R> reciprocal(Cx<R> p) { return quotient(cxone<R>(), p); }
+template <> __device__ __forceinline__ Cx<double> reciprocal(Cx<double> p) {
+  const int e = max(__double2hiint(p.x) & 0x7fffffff, __double2hiint(p.y) & 0x7fffffff) >> 20;
+  if ((unsigned)(e - (1023 - 400)) > 800u) return quotient(cxone<double>(), p);
+  const double r = rsqrt64(fma(p.x, p.x, p.y * p.y)), ir = r * r;
+  return cxmk<double>(p.x * ir, -p.y * ir);
+}
+
 template <class R> struct PanelShared {
-  R val[kPanelMaxCluster];                 // the CTAs' candidates
-  int idx[kPanelMaxCluster];
-  Cx<R> prow[kPB], jrow[kPB];              // the pivot row and row j, before the exchange
-  R wv[kPanelThreads / 32];
+  Mag<R> val[2][kPanelMaxCluster];         // the CTAs' candidates, their indices and rows
+  int idx[2][kPanelMaxCluster];
+  Cx<R> row[2][kPanelMaxCluster][kPB];
+  Cx<R> jrow[2][kPB];                      // row j before the exchange
+  Mag<R> wv[kPanelThreads / 32];
   int wi[kPanelThreads / 32];
   Cx<R> rp;
 };
@@ -88,6 +144,7 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_kernel(Cx<R>* __restri
                                                                 int32_t* __restrict__ status, int st_div, int k0, int kb,
                                                                 int rows, int slices) {
   using C_ = Cx<R>;
+  constexpr int kNone = 0x7fffffff;
   extern __shared__ __align__(16) unsigned char smraw[];
   C_* P = reinterpret_cast<C_*>(smraw);                       // (kb, rows), column by column
   __shared__ PanelShared<R> sh;
@@ -102,90 +159,89 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_kernel(Cx<R>* __restri
   const int g0 = k0 + (int)rank * rows, m = max(0, min(rows, n - g0));      // this CTA's rows g0 .. g0 + m - 1
   for (int c = warp; c < kb; c += nw)
     for (int r = lane; r < m; r += 32) P[c * rows + r] = A[g0 + r + (long long)(k0 + c) * lda];
-  __syncthreads();
   const int rstep = nt / slices, tr = tid % rstep, sl = tid / rstep;        // a thread's rows and its column slice
+  barrier_all(ctas);                                          // (and every CTA of the cluster runs)
+  Pivot<R> best = {Mag<R>::none(), kNone};
+  if (sl == 0)
+    for (int r = tr; r < m; r += rstep) best.take(Mag<R>::of(cxabs1(P[r])), g0 + r);
   for (int j = 0; j < kb; ++j) {
-    const int gj = k0 + j;
-    R best = R(-1.0);
-    int bi = 0x7fffffff;
-    for (int r = tid; r < m; r += nt) {
-      if (g0 + r < gj) continue;
-      const R v = cxabs1(P[j * rows + r]);
-      if (v > best) { best = v; bi = g0 + r; }
-    }
+    const int gj = k0 + j, buf = j & 1;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const R ov = shf(best, lane ^ o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if (lane == 0) { sh.wv[warp] = best; sh.wi[warp] = bi; }
+    for (int o = 16; o > 0; o >>= 1) best.meet(o, lane);
+    if (lane == 0) { sh.wv[warp] = best.m; sh.wi[warp] = best.i; }
     __syncthreads();
+    const int jr = gj - g0;
     if (warp == 0) {
-      best = lane < nw ? sh.wv[lane] : R(-1.0);
-      bi = lane < nw ? sh.wi[lane] : 0x7fffffff;
+      best.m = lane < nw ? sh.wv[lane] : Mag<R>::none();
+      best.i = lane < nw ? sh.wi[lane] : kNone;
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
-        const R ov = shf(best, lane ^ o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+      for (int o = 16; o > 0; o >>= 1) best.meet(o, lane);
+      if (best.m == Mag<R>::none()) best.i = kNone;
+      if (best.i != kNone && lane < kb) {
+        const C_ v = P[lane * rows + best.i - g0];
+        for (unsigned c = 0; c < ctas; ++c) put_remote(&sh.row[buf][rank][lane], c, v);
       }
       if (lane < (int)ctas) {
-        put_remote(&sh.val[rank], (unsigned)lane, best);
-        put_remote(&sh.idx[rank], (unsigned)lane, bi);
+        put_remote(&sh.val[buf][rank], (unsigned)lane, best.m);
+        put_remote(&sh.idx[buf][rank], (unsigned)lane, best.i);
       }
-    }
-    barrier_all(ctas);
-    best = sh.val[0]; bi = sh.idx[0];
-    for (unsigned c = 1; c < ctas; ++c) {
-      const R ov = sh.val[c];
-      const int oi = sh.idx[c];
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    // no finite candidate (NaN): the row itself, as a search that finds nothing larger
-    const int p = bi == 0x7fffffff ? gj : bi;
-    if (rank == 0 && tid == 0) ipiv[gj] = p;
-    // the owners send the pivot row and row j to every CTA (a warp each; lane = column)
-    const int pr = p - g0, jr = gj - g0;
-    if (warp == 0 && pr >= 0 && pr < m && lane < kb) {
-      const C_ v = P[lane * rows + pr];
-      for (unsigned c = 0; c < ctas; ++c) put_remote(&sh.prow[lane], c, v);
     }
     if (warp == 1 && jr >= 0 && jr < m && lane < kb) {
       const C_ v = P[lane * rows + jr];
-      for (unsigned c = 0; c < ctas; ++c) put_remote(&sh.jrow[lane], c, v);
+      for (unsigned c = 0; c < ctas; ++c) put_remote(&sh.jrow[buf][lane], c, v);
     }
     barrier_all(ctas);
-    const C_ piv = sh.prow[j];
+    Pivot<R> top = {sh.val[buf][0], sh.idx[buf][0]};
+    int from = 0;
+    for (unsigned c = 1; c < ctas; ++c) {
+      const int was = top.i;
+      top.take(sh.val[buf][c], sh.idx[buf][c]);
+      if (top.i != was) from = (int)c;
+    }
+    // no finite candidate (NaN): the row itself, as a search that finds nothing larger
+    const bool found = top.i != kNone;
+    const int p = found ? top.i : gj;
+    const C_* prow = found ? sh.row[buf][from] : sh.jrow[buf];
+    if (rank == 0 && tid == 0) ipiv[gj] = p;
+    const C_ piv = prow[j];
     const bool zero = piv.x == R(0.0) && piv.y == R(0.0);
+    const int pr = p - g0;
     if (p != gj) {
-      if (warp == 0 && pr >= 0 && pr < m && lane < kb) P[lane * rows + pr] = sh.jrow[lane];
-      if (warp == 1 && jr >= 0 && jr < m && lane < kb) P[lane * rows + jr] = sh.prow[lane];
+      if (warp == 0 && pr >= 0 && pr < m && lane < kb) P[lane * rows + pr] = sh.jrow[buf][lane];
+      if (warp == 1 && jr >= 0 && jr < m && lane < kb) P[lane * rows + jr] = prow[lane];
     }
-    if (zero) {
-      if (rank == 0 && tid == 0) wb_flag(st, WB_ST_SINGULAR);
-      barrier_all(ctas);
-      continue;
-    }
-    if (warp == nw - 1) {
-      const C_ r = quotient(cxone<R>(), piv);
+    if (zero && rank == 0 && tid == 0) wb_flag(st, WB_ST_SINGULAR);
+    if (!zero && warp == nw - 1) {
+      const C_ r = reciprocal(piv);
       if (lane == 0) sh.rp = r;
     }
     __syncthreads();
-    const C_ rp = sh.rp;
+    if (!zero) {
+      const C_ rp = sh.rp;
+      for (int r = tid; r < m; r += nt)
+        if (g0 + r > gj) P[j * rows + r] = mul<kScale>(P[j * rows + r], rp);
+    }
+    __syncthreads();
+    best.m = Mag<R>::none(); best.i = kNone;
     for (int r = tr; r < m; r += rstep) {
       if (g0 + r <= gj) continue;
-      const C_ l = mul<kScale>(P[j * rows + r], rp);
+      const C_ l = P[j * rows + r];
+      int c = j + 1 + sl;
+      if (sl == 0 && c < kb) {                                // column j + 1, and its search
+        C_ v = P[c * rows + r];
+        if (!zero) {
+          v = sub_mul<kUpdate>(v, l, prow[c]);
+          P[c * rows + r] = v;
+        }
+        best.take(Mag<R>::of(cxabs1(v)), g0 + r);
+        c += slices;
+      }
+      if (zero) continue;
 #pragma unroll 4
-      for (int c = j + 1 + sl; c < kb; c += slices) P[c * rows + r] = sub_mul<kUpdate>(P[c * rows + r], l, sh.prow[c]);
+      for (; c < kb; c += slices) P[c * rows + r] = sub_mul<kUpdate>(P[c * rows + r], l, prow[c]);
     }
-    __syncthreads();                                          // column j is read by all slices first
-    for (int r = tid; r < m; r += nt)
-      if (g0 + r > gj) P[j * rows + r] = mul<kScale>(P[j * rows + r], rp);
-    // (the next step's first read of column j + 1 and of sh comes after its own barriers)
-    if (ctas == 1) __syncthreads();
-    else barrier_all(ctas);
   }
+  __syncthreads();
   for (int c = warp; c < kb; c += nw)
     for (int r = lane; r < m; r += 32) A[g0 + r + (long long)(k0 + c) * lda] = P[c * rows + r];
 }
@@ -317,30 +373,33 @@ __global__ void __launch_bounds__(256) laswp_kernel(Cx<R>* __restrict__ Ball, in
 }
 
 // ------------------------------------------------------------------- a diagonal block's solve
-// op(A)'s diagonal block [i0, i0 + ib) (ib <= 64) against 16 columns a CTA: 8 threads a column, thread g
-// its rows g, g + 8, ... in registers; a solved row goes to the others by shuffles and is taken off
-// theirs at once (right-looking).
+// op(A)'s diagonal block [i0, i0 + ib) (ib <= 64) against 128 / T columns a CTA: T threads a column, thread
+// g its rows g, g + T, ... in registers; a solved row goes to the others by shuffles and is taken off
+// theirs at once (right-looking; the operations on an element and their order do not depend on T).
+// In FP64 a warp's work is FP64 issue, 1152 (T = 8), 640 (16) or 384 (32) instructions of 64 cycles for
+// 32 / T columns: the host takes the T whose rounds over the GPU's schedulers cost least.
 constexpr int kTB = 64;
 constexpr int kTriThreads = 128;
 
-template <class R>
+template <class R, int T>
 __global__ void __launch_bounds__(kTriThreads) trsm_diag_kernel(const Cx<R>* __restrict__ LUall, int lda, long long a_bs,
                                                                Cx<R>* __restrict__ Ball, int nrhs, int ldb,
                                                                long long b_bs, int i0, int ib, int lower, int unit,
                                                                int trans) {
   using C_ = Cx<R>;
+  constexpr int Q = kTB / T;
   extern __shared__ __align__(16) unsigned char smraw[];
   C_* sT = reinterpret_cast<C_*>(smraw);                      // [t][r], ld kTB + 1: element (r, t) of op(A)
   __shared__ C_ sD[kTB];                                      // reciprocal diagonal (FP64), diagonal (others)
   const C_* LU = LUall + blockIdx.y * a_bs;
   C_* B = Ball + blockIdx.y * b_bs;
-  const int tid = threadIdx.x, lane = tid & 31, g = lane & 7, first = lane & ~7;
-  const int c = (blockIdx.x * kTriThreads + tid) >> 3;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane % T, first = lane - g;
+  const int c = (blockIdx.x * kTriThreads + tid) / T;
   const bool live = c < nrhs;
   C_* col = B + i0 + (long long)(live ? c : 0) * ldb;
-  C_ x[8];
+  C_ x[Q];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) x[q] = (live && g + 8 * q < ib) ? col[g + 8 * q] : cxzero<R>();
+  for (int q = 0; q < Q; ++q) x[q] = (live && g + T * q < ib) ? col[g + T * q] : cxzero<R>();
   for (int e = tid; e < ib * ib; e += kTriThreads) {
     const int a = e % ib, b = e / ib;                         // memory order: (a, b) down a column of LU
     const C_ v = LU[i0 + a + (long long)(i0 + b) * lda];
@@ -350,16 +409,16 @@ __global__ void __launch_bounds__(kTriThreads) trsm_diag_kernel(const Cx<R>* __r
   __syncthreads();
   if (tid < ib && !unit) {
     const C_ d = sT[tid * (kTB + 1) + tid];
-    sD[tid] = sizeof(R) == 8 && !std::is_same<R, df64>::value ? quotient(cxone<R>(), d) : d;
+    sD[tid] = std::is_same<R, double>::value ? quotient(cxone<R>(), d) : d;
   }
   __syncthreads();
   constexpr bool kInv = std::is_same<R, double>::value;
   if (lower) {
 #pragma unroll
-    for (int qt = 0; qt < 8; ++qt)
+    for (int qt = 0; qt < Q; ++qt)
 #pragma unroll 1
-      for (int gt = 0; gt < 8; ++gt) {
-        const int t = 8 * qt + gt;
+      for (int gt = 0; gt < T; ++gt) {
+        const int t = T * qt + gt;
         if (t >= ib) break;
         if (!unit) {
           const C_ v = kInv ? x[qt] * sD[t] : quotient(x[qt], sD[t]);
@@ -367,16 +426,16 @@ __global__ void __launch_bounds__(kTriThreads) trsm_diag_kernel(const Cx<R>* __r
         }
         const C_ xt = shf(x[qt], first + gt);
         const C_* l = sT + t * (kTB + 1) + g;
-        if (g > gt) x[qt] = sub_mul<kUpdate>(x[qt], l[8 * qt], xt);
+        if (g > gt) x[qt] = sub_mul<kUpdate>(x[qt], l[T * qt], xt);
 #pragma unroll
-        for (int q = qt + 1; q < 8; ++q) x[q] = sub_mul<kUpdate>(x[q], l[8 * q], xt);
+        for (int q = qt + 1; q < Q; ++q) x[q] = sub_mul<kUpdate>(x[q], l[T * q], xt);
       }
   } else {
 #pragma unroll
-    for (int qt = 7; qt >= 0; --qt)
+    for (int qt = Q - 1; qt >= 0; --qt)
 #pragma unroll 1
-      for (int gt = 7; gt >= 0; --gt) {
-        const int t = 8 * qt + gt;
+      for (int gt = T - 1; gt >= 0; --gt) {
+        const int t = T * qt + gt;
         if (t >= ib) continue;
         if (!unit) {
           const C_ v = kInv ? x[qt] * sD[t] : quotient(x[qt], sD[t]);
@@ -384,14 +443,14 @@ __global__ void __launch_bounds__(kTriThreads) trsm_diag_kernel(const Cx<R>* __r
         }
         const C_ xt = shf(x[qt], first + gt);
         const C_* l = sT + t * (kTB + 1) + g;
-        if (g < gt) x[qt] = sub_mul<kUpdate>(x[qt], l[8 * qt], xt);
+        if (g < gt) x[qt] = sub_mul<kUpdate>(x[qt], l[T * qt], xt);
 #pragma unroll
-        for (int q = 0; q < qt; ++q) x[q] = sub_mul<kUpdate>(x[q], l[8 * q], xt);
+        for (int q = 0; q < qt; ++q) x[q] = sub_mul<kUpdate>(x[q], l[T * q], xt);
       }
   }
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
-    if (live && g + 8 * q < ib) col[g + 8 * q] = x[q];
+  for (int q = 0; q < Q; ++q)
+    if (live && g + T * q < ib) col[g + T * q] = x[q];
 }
 
 // The upper solve in FP32: the row's sum runs over the later unknowns in ascending order, so its first
