@@ -801,64 +801,103 @@ __global__ void __launch_bounds__(256) group_product_kernel(const cplx* __restri
   }
 }
 
-// One CTA per pair: d, the groups (lock-free union-find over the strong couplings, links always
-// from the larger root index to the smaller, retries bounded), the group blocks into slots, E and
-// the new lambda. A pair whose groups do not fit (more than kGroupMax members, slots exhausted,
-// union retries exhausted) is flagged WB_ST_NOCONV.
-__global__ void __launch_bounds__(256) group_kernel(int n, const Cx<float>* __restrict__ Gall, cplx* __restrict__ lam_all,
-                                                    Cx<float>* __restrict__ Eall, GroupBufs gb, int32_t* __restrict__ status,
-                                                    int st_div) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cplx* d = reinterpret_cast<cplx*>(smraw);
-  int* parent = reinterpret_cast<int*>(d + n);
-  int* label = parent + n;
-  int* cnt = label + n;
-  int* slot = cnt + n;
-  int* fill = slot + n;
-  __shared__ int s_fail;
+// The groups of a pair, in four launches: d and its scale; the links (lock-free union-find over the strong
+// couplings, always from the larger root index to the smaller, retries bounded); the groups' blocks into
+// slots; E and the new lambda. Links and E look at all n^2 entries with moduli and divisions in FP64, a
+// scheduler's 64 cycles an instruction, and are spread over the GPU (one CTA a pair took 18 ms at n = 798);
+// the links first rule a coupling out in FP32. A pair whose groups do not fit (more than kGroupMax members,
+// slots exhausted, union retries exhausted) is flagged WB_ST_NOCONV.
+//
+// Scratch a pair: d (n), and parent (n), label (n), scale as a double.
+struct GroupScratch {
+  cplx* d; int* ints; long long stride;                       // both 16 `stride` bytes a pair
+  __device__ __forceinline__ cplx* dd(int p) const { return d + p * stride; }
+  __device__ __forceinline__ int* parent(int p) const { return ints + 4 * p * stride; }
+  __device__ __forceinline__ double* scale(int p, int n) const { return reinterpret_cast<double*>(parent(p) + 2 * n); }
+};
+
+__global__ void __launch_bounds__(256) group_d_kernel(int n, const Cx<float>* __restrict__ Gall, const cplx* __restrict__ lam_all,
+                                                      GroupScratch gs) {
   __shared__ double s_red[32];
   const int p = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const long long n2 = (long long)n * n;
-  const Cx<float>* G = Gall + p * n2;
-  Cx<float>* E = Eall + p * n2;
-  cplx* lam = lam_all + (long long)p * n;
-  if (tid == 0) s_fail = 0;
+  const Cx<float>* G = Gall + p * ((long long)n * n);
+  cplx* d = gs.dd(p);
+  int* parent = gs.parent(p);
   double mx = 0.0;
   for (int i = tid; i < n; i += blockDim.x) {
     const Cx<float> g = G[i + (long long)i * n];
-    const cplx v = cadd(lam[i], cmk((double)g.x, (double)g.y));
-    d[i] = v; parent[i] = i; cnt[i] = 0; slot[i] = -1; fill[i] = 0;
+    const cplx v = cadd(lam_all[(long long)p * n + i], cmk((double)g.x, (double)g.y));
+    d[i] = v; parent[i] = i;
     mx = fmax(mx, cabsv(v));
   }
   for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   if (lane == 0) s_red[warp] = mx;
   __syncthreads();
-  double scale = 0.0;
-  for (int k = 0; k < nw; ++k) scale = fmax(scale, s_red[k]);
-  volatile int* vp = parent;
-  for (long long e = tid; e < n2; e += blockDim.x) {
-    const int i = (int)(e % n), j = (int)(e / n);
-    if (i == j) continue;
-    const Cx<float> g = G[e];
-    const double ga = hypot((double)g.x, (double)g.y);
-    if (!(ga > kCouple * cabsv(csub(d[j], d[i])))) continue;
-    int a = i, b = j;
-    bool linked = false;
-    for (int tries = 0; tries < 64 + 4 * n && !linked; ++tries) {
-      int ra = a, rb = b;
-      for (int h = 0; h < n && vp[ra] != ra; ++h) ra = vp[ra];
-      for (int h = 0; h < n && vp[rb] != rb; ++h) rb = vp[rb];
-      if (ra == rb) { linked = true; break; }
-      if (ra > rb) { const int t = ra; ra = rb; rb = t; }
-      if (atomicCAS(&parent[rb], rb, ra) == rb) linked = true;
-    }
-    if (!linked) s_fail = 1;
+  if (tid == 0) {
+    double scale = 0.0;
+    for (int k = 0; k < nw; ++k) scale = fmax(scale, s_red[k]);
+    *gs.scale(p, n) = scale;
   }
+}
+
+// a warp a column
+__global__ void __launch_bounds__(256) group_link_kernel(int n, const Cx<float>* __restrict__ Gall, GroupScratch gs,
+                                                         int32_t* __restrict__ status, int st_div) {
+  const int p = blockIdx.y, lane = threadIdx.x & 31, warps = gridDim.x * 8;
+  const Cx<float>* G = Gall + p * ((long long)n * n);
+  const cplx* d = gs.dd(p);
+  int* parent = gs.parent(p);
+  volatile int* vp = parent;
+  for (int j = blockIdx.x * 8 + (threadIdx.x >> 5); j < n; j += warps) {
+    const cplx dj = d[j];
+    for (int i = lane; i < n; i += 32) {
+      if (i == j) continue;
+      const Cx<float> g = G[i + (long long)j * n];
+      const cplx df = csub(dj, d[i]);
+      // |g| <= sqrt(2) max(|re|, |im|), |d_j - d_i| >= max(..): no squares, so nothing leaves FP32's range
+      const float gm = fmaxf(fabsf(g.x), fabsf(g.y)), dm = fmaxf(fabsf((float)df.x), fabsf((float)df.y));
+      if (gm * 1.41422f <= (float)kCouple * 0.9999f * dm && dm > 1e-30f && gm < 1e30f) continue;
+      const double ga = hypot((double)g.x, (double)g.y);
+      if (!(ga > kCouple * cabsv(df))) continue;
+      int a = i, b = j;
+      bool linked = false;
+      for (int tries = 0; tries < 64 + 4 * n && !linked; ++tries) {
+        int ra = a, rb = b;
+        for (int h = 0; h < n && vp[ra] != ra; ++h) ra = vp[ra];
+        for (int h = 0; h < n && vp[rb] != rb; ++h) rb = vp[rb];
+        if (ra == rb) { linked = true; break; }
+        if (ra > rb) { const int t = ra; ra = rb; rb = t; }
+        if (atomicCAS(&parent[rb], rb, ra) == rb) linked = true;
+      }
+      if (!linked) wb_flag(status + p / st_div, WB_ST_NOCONV);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) group_kernel(int n, const Cx<float>* __restrict__ Gall, const cplx* __restrict__ lam_all,
+                                                    GroupBufs gb, GroupScratch gs, int32_t* __restrict__ status,
+                                                    int st_div) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  int* label = reinterpret_cast<int*>(smraw);
+  int* cnt = label + n;
+  int* slot = cnt + n;
+  int* fill = slot + n;
+  __shared__ int s_fail;
+  const int p = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const long long n2 = (long long)n * n;
+  const Cx<float>* G = Gall + p * n2;
+  const cplx* lam = lam_all + (long long)p * n;
+  const int* parent = gs.parent(p);
+  int* glabel = gs.parent(p) + n;
+  const double scale = *gs.scale(p, n);
+  if (tid == 0) s_fail = 0;
+  for (int i = tid; i < n; i += blockDim.x) { cnt[i] = 0; slot[i] = -1; fill[i] = 0; }
   __syncthreads();
   for (int i = tid; i < n; i += blockDim.x) {
     int r = i;
-    for (int h = 0; h < n && vp[r] != r; ++h) r = vp[r];
+    for (int h = 0; h < n && parent[r] != r; ++h) r = parent[r];
     label[i] = r;
+    glabel[i] = r;
     atomicAdd(&cnt[r], 1);
   }
   __syncthreads();
@@ -924,23 +963,37 @@ __global__ void __launch_bounds__(256) group_kernel(int n, const Cx<float>* __re
     for (int o = 16; o > 0; o >>= 1) off = fmax(off, __shfl_xor_sync(0xffffffffu, off, o));
     if (lane == 0) gb.offmax[sl] = off / (scale > 0.0 ? scale : 1.0);
   }
-  // first-order corrections between groups, and the new eigenvalues
-  for (long long e = tid; e < n2; e += blockDim.x) {
-    const int i = (int)(e % n), j = (int)(e / n);
-    Cx<float> v = cxzero<float>();
-    if (i != j && label[i] != label[j]) {
-      const cplx dd = csub(d[j], d[i]);
-      if (dd.x != 0.0 || dd.y != 0.0) {
-        const Cx<float> g = G[e];
-        const cplx q = cdiv(cmk((double)g.x, (double)g.y), dd);
-        v = cxmk<float>((float)q.x, (float)q.y);
-      }
-    }
-    E[e] = v;
-  }
   __syncthreads();
-  for (int i = tid; i < n; i += blockDim.x) lam[i] = d[i];
   if (tid == 0 && s_fail) wb_flag(status + p / st_div, WB_ST_NOCONV);
+}
+
+// first-order corrections between groups, and the new eigenvalues; a warp a column
+__global__ void __launch_bounds__(256) group_correct_kernel(int n, const Cx<float>* __restrict__ Gall, cplx* __restrict__ lam_all,
+                                                            Cx<float>* __restrict__ Eall, GroupScratch gs) {
+  const int p = blockIdx.y, lane = threadIdx.x & 31, warps = gridDim.x * 8;
+  const long long n2 = (long long)n * n;
+  const Cx<float>* G = Gall + p * n2;
+  Cx<float>* E = Eall + p * n2;
+  const cplx* d = gs.dd(p);
+  const int* label = gs.parent(p) + n;
+  for (int j = blockIdx.x * 8 + (threadIdx.x >> 5); j < n; j += warps) {
+    const cplx dj = d[j];
+    const int lj = label[j];
+    for (int i = lane; i < n; i += 32) {
+      const long long e = i + (long long)j * n;
+      Cx<float> v = cxzero<float>();
+      if (i != j && label[i] != lj) {
+        const cplx dd = csub(dj, d[i]);
+        if (dd.x != 0.0 || dd.y != 0.0) {
+          const Cx<float> g = G[e];
+          const cplx q = cdiv(cmk((double)g.x, (double)g.y), dd);
+          v = cxmk<float>((float)q.x, (float)q.y);
+        }
+      }
+      E[e] = v;
+    }
+    if (lane == 0) lam_all[(long long)p * n + j] = dj;
+  }
 }
 
 // One CTA per used slot: rotate the group's columns of W by the block's eigenvectors and set
@@ -1087,7 +1140,9 @@ void stage_b_newton(cudaStream_t s, int P, int N, const cplx* conv, const int* p
   Cx<double>* Sm = (Cx<double>*)nb.F3;
   Cx<double>* Ym = (Cx<double>*)Vd;
   const Cx<double>* cv = (const Cx<double>*)conv;
-  const size_t gsm = (size_t)n * (sizeof(cplx) + 5 * sizeof(int));
+  const size_t gsm = (size_t)n * 4 * sizeof(int);
+  const GroupScratch gs = {(cplx*)Tm, (int*)Um, Nn};             // T and U are free between the residual and the next product
+  const dim3 gcols((unsigned)max(1LL, min((long long)(n + 7) / 8, (16LL * sm_count() + P - 1) / P)), (unsigned)P);
   cudaFuncSetAttribute(group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm);
   for (int it = 0; it < kNewtonSteps; ++it) {
     if (it > 0) convert<double, float>(s, (const Cx<double>*)Wd, nb.F1, tot);
@@ -1107,7 +1162,10 @@ void stage_b_newton(cudaStream_t s, int P, int N, const cplx* conv, const int* p
     note_launch();
     getrs<float>(s, P, n, nb.F1, n, n2, nb.piv, n, nb.F4, n, n, n2, 0);            // G = W32^-1 R
     cudaMemsetAsync(gb.count, 0, 2 * sizeof(int), s);
-    group_kernel<<<P, 256, gsm, s>>>(n, nb.F4, nb.lam, nb.F3, gb, st, st_div); note_launch();
+    group_d_kernel<<<P, 256, 0, s>>>(n, nb.F4, nb.lam, gs); note_launch();
+    group_link_kernel<<<gcols, 256, 0, s>>>(n, nb.F4, gs, st, st_div); note_launch();
+    group_kernel<<<P, 256, gsm, s>>>(n, nb.F4, nb.lam, gb, gs, st, st_div); note_launch();
+    group_correct_kernel<<<gcols, 256, 0, s>>>(n, nb.F4, nb.lam, nb.F3, gs); note_launch();
     gemm<float>(s, P, n, n, n, one, nb.F2, 1, n, n2, nb.F3, 1, n, n2, zero, nb.F4, 1, n, n2);   // W E
     accumulate_kernel<float, double><<<nblk(tot, 256), 256, 0, s>>>(tot, nb.F4, (Cx<double>*)Wd); note_launch();
     // exact diagonalisation of the groups
