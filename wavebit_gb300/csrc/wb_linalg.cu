@@ -568,6 +568,8 @@ void getrf(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a_bs, 
     return;
   }
   int width = LU_PB;
+  // FP64: equal panels, so that no product is a few rows deep or wide and falls off the tensor cores
+  if (fp64) { const int panels = (n + LU_PB - 1) / LU_PB; width = (n + panels - 1) / panels; }
   while (width > 8 && panel_shape<R>(batch, n, width).smem > 212 * 1024) width /= 2;
   cudaFuncSetAttribute(tri::lu_panel_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024);
   for (int k0 = 0; k0 < n; k0 += width) {
@@ -767,10 +769,10 @@ static bool getrs_narrow(cudaStream_t s, int batch, int n, const Cx<R>* LU, int 
 
 // Many right-hand sides: a blocked substitution across the GPU. The FP32 form's cascade and the FP64
 // form take it, the latter with its products on the tensor cores.
-// The row interchanges are applied first (trans 0) or last (trans 1); then, per block of TB_NB rows, the
+// The row interchanges are applied first (trans 0) or last (trans 1); then, per block of at most TB_NB rows, the
 // diagonal block is solved for every column (tri::trsm_diag_kernel, in FP32's upper solve
 // trsm_upper_f32_kernel) and the batched GEMM subtracts the block's contribution from the rows still to
-// solve (K = TB_NB). The substitution order and pivots are those of getrs_kernel; only the summation
+// solve. The substitution order and pivots are those of getrs_kernel; only the summation
 // order differs. A diagonal block of 450 columns: FP64 400 -> 80 us, FP32 65 -> 20 us.
 constexpr int TB_NB = tri::kTB;
 
@@ -818,9 +820,13 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
     note_launch();
   };
   const double2 m1 = make_double2(-1.0, 0.0), p1 = make_double2(1.0, 0.0);
+  // FP64: equal blocks (at n = 450 the last of 64 has two rows, and its two products took 270 us each on
+  // the FP64 pipes); FP32 keeps its order of summation
+  int nb = TB_NB;
+  if (std::is_same<R, double>::value) { const int blocks = (n + TB_NB - 1) / TB_NB; nb = (n + blocks - 1) / blocks; }
   // forward: L (unit lower) for trans 0, U^T (lower, stored diagonal) for trans 1
-  for (int i0 = 0; i0 < n; i0 += TB_NB) {
-    const int ib = min(TB_NB, n - i0), i1 = i0 + ib, m = n - i1;
+  for (int i0 = 0; i0 < n; i0 += nb) {
+    const int ib = min(nb, n - i0), i1 = i0 + ib, m = n - i1;
     diagonal(i0, ib, 1, trans == 0);
     if (m > 0) {
       if (trans == 0)
@@ -832,8 +838,8 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
     }
   }
   // backward: U (upper, stored diagonal) for trans 0, L^T (unit upper) for trans 1
-  for (int i1 = n; i1 > 0; i1 -= TB_NB) {
-    const int i0 = max(0, i1 - TB_NB), ib = i1 - i0;
+  for (int i1 = n; i1 > 0; i1 -= nb) {
+    const int i0 = max(0, i1 - nb), ib = i1 - i0;
     diagonal(i0, ib, 0, trans == 1);
     if (i0 > 0) {
       if (trans == 0)
