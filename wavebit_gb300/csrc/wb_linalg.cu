@@ -207,6 +207,8 @@ void gemm_idx(cudaStream_t s, int batch, int m, int n, int k, double2 alpha,
 // at a unit roundoff of about 2^-48 (the error grows like K 2^-48 of sum |a||b| in the worst case).
 // Used by the mixed form for the products whose results must be FP64-accurate (the Newton
 // residual Omega^2 W and V = Omega_R W), never by the plain FP64 form.
+// Bound by FP32 issue; two CTAs an SM (128 registers, so the loop over a tile's k is not unrolled) hide
+// one another's latencies: 32 x 4 matrices at n = 450 8.7 -> 7.2 ms a product.
 namespace {
 struct DD { float hi, lo; };
 __device__ __forceinline__ void dd_mac(DD& acc, float ah, float al, float bh, float bl) {
@@ -225,14 +227,34 @@ __device__ __forceinline__ void dd_norm(DD& a) {
   a.lo = __fsub_rn(a.lo, __fsub_rn(s, a.hi));
   a.hi = s;
 }
+// x as hi + lo, both rounded to nearest even: by integer operations on the double's bits, since the two
+// conversions each way and the subtraction hold a scheduler for 64 cycles each (as much again as a third of
+// a tile's products). lo is (signed remainder below hi's last bit) 2^(e - 1075); zero, and what leaves FP32's
+// range with lo, goes by the conversions.
+__device__ __forceinline__ float2 dd_split(double x) {
+  const int h = __double2hiint(x);
+  const unsigned l = (unsigned)__double2loint(x);
+  const int e = (h >> 20) & 0x7ff;
+  if ((unsigned)(e - 960) > 180u) {
+    const float hi = (float)x;
+    return make_float2(hi, (float)(x - (double)hi));
+  }
+  const unsigned sign = (unsigned)h & 0x80000000u;
+  const unsigned top = ((unsigned)(h & 0xfffff) << 3) | (l >> 29), low = l & 0x1fffffffu;
+  const unsigned up = (low + (top & 1u)) > 0x10000000u ? 1u : 0u;
+  const float hi = __uint_as_float(sign | ((((unsigned)(e - 896) << 23) | top) + up));
+  int rem = (int)low - (int)(up << 29);
+  rem = sign ? -rem : rem;
+  return make_float2(hi, (float)rem * __uint_as_float((unsigned)(e - 1075 + 127) << 23));
+}
 // (re.hi, re.lo, im.hi, im.lo) of an FP64 complex value
 __device__ __forceinline__ float4 dd_split(double2 v) {
-  const float rh = (float)v.x, ih = (float)v.y;
-  return make_float4(rh, (float)(v.x - (double)rh), ih, (float)(v.y - (double)ih));
+  const float2 a = dd_split(v.x), b = dd_split(v.y);
+  return make_float4(a.x, a.y, b.x, b.y);
 }
 }  // namespace
 
-__global__ void __launch_bounds__(256) gemm_dd_kernel(
+__global__ void __launch_bounds__(256, 2) gemm_dd_kernel(
     int m, int n, int k, double2 alpha, const double2* __restrict__ A, long long a_rs, long long a_cs,
     long long a_bs, const int* __restrict__ a_idx, const double2* __restrict__ B, long long b_rs, long long b_cs,
     long long b_bs, double2 beta, double2* __restrict__ C, long long c_rs, long long c_cs, long long c_bs) {
@@ -264,7 +286,7 @@ __global__ void __launch_bounds__(256) gemm_dd_kernel(
       sB[r][c] = (gr < k && gc < n) ? dd_split(B[gr * b_rs + gc * b_cs]) : zero4;
     }
     __syncthreads();
-#pragma unroll
+#pragma unroll 1
     for (int kk = 0; kk < GK; ++kk) {
       float4 a[4], b[4];
 #pragma unroll
@@ -767,6 +789,44 @@ static bool getrs_narrow(cudaStream_t s, int batch, int n, const Cx<R>* LU, int 
   return true;
 }
 
+// B[r, :] -= op(A)(r, :) X for the few columns of a transposed FP64 solve: row r of A^T is column r of A, so
+// a warp takes a row and its lanes run down that column. (The tiled product spends 270 us on 3 columns.)
+template <int NC>
+__global__ void __launch_bounds__(256) trans_update_kernel(const Cx<double>* __restrict__ LUall, int lda, long long a_bs,
+                                                           Cx<double>* __restrict__ Ball, int nrhs, int ldb,
+                                                           long long b_bs, int i0, int ib, int r0, int m) {
+  const int lane = threadIdx.x & 31, r = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= m) return;
+  const Cx<double>* a = LUall + blockIdx.y * a_bs + i0 + (long long)(r0 + r) * lda;
+  Cx<double>* B = Ball + blockIdx.y * b_bs;
+  double sx[NC], sy[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) sx[c] = sy[c] = 0.0;
+  for (int k = lane; k < ib; k += 32) {
+    const Cx<double> v = a[k];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+      if (c < nrhs) {
+        const Cx<double> x = B[i0 + k + (long long)c * ldb];
+        sx[c] = fma(v.x, x.x, fma(-v.y, x.y, sx[c]));
+        sy[c] = fma(v.x, x.y, fma(v.y, x.x, sy[c]));
+      }
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    if (c >= nrhs) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sx[c] += __shfl_xor_sync(0xffffffffu, sx[c], o);
+      sy[c] += __shfl_xor_sync(0xffffffffu, sy[c], o);
+    }
+    if (lane == 0) {
+      Cx<double>* b = B + r0 + r + (long long)c * ldb;
+      *b = cxmk<double>(b->x - sx[c], b->y - sy[c]);
+    }
+  }
+}
+
 // Many right-hand sides: a blocked substitution across the GPU. The FP32 form's cascade and the FP64
 // form take it, the latter with its products on the tensor cores.
 // The row interchanges are applied first (trans 0) or last (trans 1); then, per block of at most TB_NB rows, the
@@ -824,11 +884,21 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
   // the FP64 pipes); FP32 keeps its order of summation
   int nb = TB_NB;
   if (std::is_same<R, double>::value) { const int blocks = (n + TB_NB - 1) / TB_NB; nb = (n + blocks - 1) / blocks; }
+  // few columns of a transposed solve: the rows [r0, r0 + m) less the block [i0, i0 + ib)'s part
+  auto few = [&](int i0, int ib, int r0, int m) {
+    if constexpr (std::is_same<R, double>::value) {
+      if (!trans || nrhs >= 8) return false;
+      trans_update_kernel<7><<<dim3((m + 7) / 8, batch), 256, 0, s>>>(LU, lda, a_bs, B, nrhs, ldb, b_bs, i0, ib, r0, m);
+      note_launch();
+      return true;
+    }
+    return false;
+  };
   // forward: L (unit lower) for trans 0, U^T (lower, stored diagonal) for trans 1
   for (int i0 = 0; i0 < n; i0 += nb) {
     const int ib = min(nb, n - i0), i1 = i0 + ib, m = n - i1;
     diagonal(i0, ib, 1, trans == 0);
-    if (m > 0) {
+    if (m > 0 && !few(i0, ib, i1, m)) {
       if (trans == 0)
         gemm<R>(s, batch, m, nrhs, ib, m1, LU + i1 + (long long)i0 * lda, 1, lda, a_bs, B + i0, 1, ldb, b_bs, p1,
                 B + i1, 1, ldb, b_bs);
@@ -841,7 +911,7 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
   for (int i1 = n; i1 > 0; i1 -= nb) {
     const int i0 = max(0, i1 - nb), ib = i1 - i0;
     diagonal(i0, ib, 0, trans == 1);
-    if (i0 > 0) {
+    if (i0 > 0 && !few(i0, ib, 0, i0)) {
       if (trans == 0)
         gemm<R>(s, batch, i0, nrhs, ib, m1, LU + (long long)i0 * lda, 1, lda, a_bs, B + i0, 1, ldb, b_bs, p1, B, 1,
                 ldb, b_bs);
