@@ -208,6 +208,7 @@ __device__ __forceinline__ Cx<double> wilkinson(Cx<double> p, Cx<double> u1, Cx<
 // Reflector of (alpha, x) with x real, as used by the chase: beta = -sign(Re alpha)|(alpha, x)|,
 // tau = (beta - alpha)/beta, v2 = x/(alpha - beta); one square root and two reciprocals.
 template <class R> struct Rot { Cx<R> t1, v2; R t2, beta; bool identity; };
+// Called by a whole warp with the same values in every lane.
 template <class R> __device__ __forceinline__ Rot<R> householder(Cx<R> alpha, R x) {
   Rot<R> r;
   // scaled by m = max(|Re a|, |Im a|, |x|) so that squares stay in range (the double-float form
@@ -221,9 +222,19 @@ template <class R> __device__ __forceinline__ Rot<R> householder(Cx<R> alpha, R 
   const R ax = qr::plain_mul(alpha.x, im), ay = qr::plain_mul(alpha.y, im), xs = qr::plain_mul(x, im);
   R nrm = rsqrt_(qr::sum_squares(ax, ay, xs));
   R bs = (ax >= R(0.0)) ? -nrm : nrm;                         // beta / m
-  R ib = R(1.0) / bs;
   Cx<R> d = cxmk<R>(qr::plain_sub(ax, bs), ay);                              // (alpha - beta) / m
-  R idd = R(1.0) / qr::sum_squares2(d.x, d.y);
+  const R dd = qr::sum_squares2(d.x, d.y);
+  R ib, idd;
+  if constexpr (sizeof(R) == 4) {
+    // one reciprocal a half of the warp: the two are a subroutine each and would run one after the other
+    const bool upper = threadIdx.x & 16;
+    const R r = R(1.0) / (upper ? dd : bs), o = __shfl_xor_sync(0xffffffffu, r, 16);
+    ib = upper ? o : r;
+    idd = upper ? r : o;
+  } else {
+    ib = R(1.0) / bs;
+    idd = R(1.0) / dd;
+  }
   r.identity = false;
   r.beta = bs * m;
   r.t1 = cxmk<R>(qr::plain_sub(bs, ax) * ib, -(ay * ib));
