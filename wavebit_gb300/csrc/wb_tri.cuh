@@ -191,13 +191,11 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_kernel(Cx<R>* __restri
       for (unsigned c = 0; c < ctas; ++c) put_remote(&sh.jrow[buf][lane], c, v);
     }
     barrier_all(ctas);
-    Pivot<R> top = {sh.val[buf][0], sh.idx[buf][0]};
-    int from = 0;
-    for (unsigned c = 1; c < ctas; ++c) {
-      const int was = top.i;
-      top.take(sh.val[buf][c], sh.idx[buf][c]);
-      if (top.i != was) from = (int)c;
-    }
+    const int cand = (lane & (kPanelMaxCluster - 1)) % (int)ctas;
+    Pivot<R> top = {sh.val[buf][cand], sh.idx[buf][cand]};
+#pragma unroll
+    for (int o = kPanelMaxCluster / 2; o > 0; o >>= 1) top.meet(o, lane);
+    const int from = (top.i - k0) / rows;                     // the CTA with that row
     // no finite candidate (NaN): the row itself, as a search that finds nothing larger
     const bool found = top.i != kNone;
     const int p = found ? top.i : gj;
@@ -400,16 +398,24 @@ __global__ void __launch_bounds__(kTriThreads) trsm_diag_kernel(const Cx<R>* __r
   C_ x[Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) x[q] = (live && g + T * q < ib) ? col[g + T * q] : cxzero<R>();
-  for (int e = tid; e < ib * ib; e += kTriThreads) {
-    const int a = e % ib, b = e / ib;                         // memory order: (a, b) down a column of LU
-    const C_ v = LU[i0 + a + (long long)(i0 + b) * lda];
-    if (trans) sT[a * (kTB + 1) + b] = v;                     // op(A)(b, a)
-    else sT[b * (kTB + 1) + a] = v;                           // op(A)(a, b)
+#pragma unroll
+  for (int b0 = 0; b0 < kTB; b0 += 16) {                      // a warp four columns of LU, eight loads in flight
+    C_ v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int a = lane + 32 * (u & 1), b = b0 + (tid >> 5) + 4 * (u >> 1);
+      if (a < ib && b < ib) v[u] = LU[i0 + a + (long long)(i0 + b) * lda];
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int a = lane + 32 * (u & 1), b = b0 + (tid >> 5) + 4 * (u >> 1);
+      if (a < ib && b < ib) sT[trans ? a * (kTB + 1) + b : b * (kTB + 1) + a] = v[u];   // op(A)(b, a) or (a, b)
+    }
   }
   __syncthreads();
   if (tid < ib && !unit) {
     const C_ d = sT[tid * (kTB + 1) + tid];
-    sD[tid] = std::is_same<R, double>::value ? quotient(cxone<R>(), d) : d;
+    sD[tid] = std::is_same<R, double>::value ? reciprocal(d) : d;
   }
   __syncthreads();
   constexpr bool kInv = std::is_same<R, double>::value;
