@@ -392,6 +392,198 @@ __global__ void __launch_bounds__(1024) gehrd_panel_kernel(Cx<R>* __restrict__ A
   }
 }
 
+// The same panel by a cluster of CTAs a matrix, its rows shared out: one CTA pulls the trailing matrix through
+// one SM once a column (21 of a column's 45 us at n = 798) and runs the panel's products on its latencies.
+// Every CTA has the column and its reflector whole, its own rows of V and Y in shared memory, and the columns
+// l = rank, rank + ctas, .. of V whole; rows of b, and the sums V^H b and V^H v, go to all by shared memory of
+// the cluster. A row of A v is four threads, one a partial sum. Every sum has the order of gehrd_panel_kernel
+// (the norm's that of its `vthreads` threads), so the bits are its.
+constexpr int kHrdClusterThreads = 512;
+static size_t hrd_panel_shared(int n, int ctas) {
+  const int rp = (n + ctas - 1) / ctas;
+  return sizeof(Cx<float>) * ((size_t)2 * n + (size_t)2 * kHrdPanel * rp + (size_t)(kHrdPanel / ctas) * n);
+}
+
+__device__ __forceinline__ void send32(Cx<float>* p, Cx<float> v, unsigned ctas) {
+  const unsigned src = (unsigned)__cvta_generic_to_shared(p);
+  for (unsigned c = 0; c < ctas; ++c) {
+    unsigned dst;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(src), "r"(c));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(v.x) : "memory");
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + 4), "f"(v.y) : "memory");
+  }
+}
+
+__global__ void __launch_bounds__(kHrdClusterThreads) gehrd_panel_cluster_kernel(
+    Cx<float>* __restrict__ Aall, int n, int lda, long long a_bs, Cx<float>* __restrict__ tau_all, int k, int bb,
+    Cx<float>* __restrict__ Wsall, long long ws_bs, int vthreads) {
+  using R = float;
+  using C_ = Cx<float>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const unsigned ctas = qr::cta_count(), rank = qr::cta_rank();
+  const int rp = (n + (int)ctas - 1) / (int)ctas, r0 = (int)rank * rp, rows = max(0, min(rp, n - r0));
+  C_* sb = reinterpret_cast<C_*>(smraw);          // (n) the column being reduced
+  C_* sv = sb + n;                                 // (n) its reflector
+  C_* sV = sv + n;                                 // [kHrdPanel][rp] this CTA's rows
+  C_* sY = sV + kHrdPanel * rp;
+  C_* sF = sY + kHrdPanel * rp;                    // [kHrdPanel / ctas][n] whole columns of V
+  __shared__ C_ T[kHrdPanel][kHrdPanel + 1];
+  __shared__ C_ top[kHrdPanel][kHrdPanel];         // [l][i]: V(k + i, l)
+  __shared__ C_ s_vc[kHrdPanel], s_w[kHrdPanel], s_u[kHrdPanel];
+  __shared__ R red[32];
+  __shared__ C_ s_tau, s_scale;
+  __shared__ R s_beta;
+  __shared__ int s_id;
+  C_* A = Aall + (blockIdx.x / ctas) * a_bs;
+  C_* tau = tau_all + (long long)(blockIdx.x / ctas) * n;
+  C_* ws = Wsall + (blockIdx.x / ctas) * ws_bs;
+  const long long nB = (long long)n * kHrdPanel;
+  C_* V = ws;
+  C_* Vc = ws + nB;
+  C_* Y = ws + 2 * nB;
+  C_* TH = ws + 5 * nB;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+  for (int e = tid; e < kHrdPanel * (kHrdPanel + 1); e += nt) T[e / (kHrdPanel + 1)][e % (kHrdPanel + 1)] = cxzero<R>();
+  qr::barrier_all(ctas);
+  for (int j = 0; j < bb; ++j) {
+    const int c = k + j;
+    if (tid < j) s_vc[tid] = cxconj(top[tid][j]);
+    __syncthreads();
+    // b = a_c - Y_j conj(V_j(c, :))
+    for (int i = tid; i < rows; i += nt) {
+      C_ acc = A[r0 + i + (long long)c * lda];
+      for (int l = 0; l < j; ++l) acc = acc - sY[l * rp + i] * s_vc[l];
+      send32(sb + r0 + i, acc, ctas);
+    }
+    qr::barrier_all(ctas);
+    if (j > 0) {
+      // w = V_j^H b (rows below k), u = T_j^H w, b <- b - V_j u
+      for (int l = (int)rank + warp * (int)ctas; l < j; l += nw * (int)ctas) {
+        const C_* f = sF + (l / (int)ctas) * n;
+        C_ acc = cxzero<R>();
+        for (int r = k + 1 + lane; r < n; r += 32) acc = cxfma_conj(f[r], sb[r], acc);
+        acc.x = warp_sum(acc.x);
+        acc.y = warp_sum(acc.y);
+        if (lane == 0) send32(s_w + l, acc, ctas);
+      }
+      qr::barrier_all(ctas);
+      if (tid < j) {
+        C_ acc = cxzero<R>();
+        for (int lp = 0; lp <= tid; ++lp) acc = cxfma_conj(T[lp][tid], s_w[lp], acc);
+        s_u[tid] = acc;
+      }
+      __syncthreads();
+      for (int i = tid; i < rows; i += nt) {
+        if (r0 + i < k + 1) continue;
+        C_ acc = sb[r0 + i];
+        for (int l = 0; l < j; ++l) acc = acc - sV[l * rp + i] * s_u[l];
+        send32(sb + r0 + i, acc, ctas);
+      }
+      qr::barrier_all(ctas);
+    }
+    // the reflector of (b[c+1]; b[c+2:])
+    for (int vw = warp; vw < vthreads / 32; vw += nw) {
+      R part = R(0.0);
+      for (int r = c + 2 + 32 * vw + lane; r < n; r += vthreads) part = part + cxabs2(sb[r]);
+      part = warp_sum(part);
+      if (lane == 0) red[vw] = part;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      R xn2 = R(0.0);
+      for (int w = 0; w < vthreads / 32; ++w) xn2 = xn2 + red[w];
+      const Refl<R> rf = make_reflector(sb[c + 1], rsqrt_(xn2));
+      s_id = rf.identity ? 1 : 0;
+      s_tau = rf.identity ? cxzero<R>() : rf.tau;
+      s_scale = rf.scale;
+      s_beta = rf.beta;
+      if (rank == 0) tau[c] = s_tau;
+    }
+    __syncthreads();
+    const bool ident = s_id != 0;
+    const C_ tj = s_tau, scl = s_scale;
+    // v whole, V[:, j] and conj(V[:, j]), and column c in its final form
+    const bool keep = j % (int)ctas == (int)rank;
+    for (int r = tid; r < n; r += nt) {
+      C_ v = cxzero<R>();
+      if (!ident) {
+        if (r == c + 1) v = cxone<R>();
+        else if (r > c + 1) v = sb[r] * scl;
+      }
+      sv[r] = v;
+      if (keep) sF[(j / (int)ctas) * n + r] = v;
+      if (r >= k && r < k + kHrdPanel) top[j][r - k] = v;
+      const int i = r - r0;
+      if (i >= 0 && i < rows) {
+        sV[j * rp + i] = v;
+        V[r + (long long)j * n] = v;
+        Vc[r + (long long)j * n] = cxconj(v);
+        C_ a = sb[r];
+        if (!ident && r == c + 1) a = cxmk<R>(s_beta, R(0.0));
+        else if (!ident && r > c + 1) a = v;
+        A[r + (long long)c * lda] = a;
+      }
+    }
+    __syncthreads();
+    // w2 = V_j^H v, T[:j, j] = -tau T_j w2, T[j, j] = tau
+    if (j > 0) {
+      for (int l = (int)rank + warp * (int)ctas; l < j; l += nw * (int)ctas) {
+        const C_* f = sF + (l / (int)ctas) * n;
+        C_ acc = cxzero<R>();
+        for (int r = c + 1 + lane; r < n; r += 32) acc = cxfma_conj(f[r], sv[r], acc);
+        acc.x = warp_sum(acc.x);
+        acc.y = warp_sum(acc.y);
+        if (lane == 0) send32(s_w + l, acc, ctas);
+      }
+    }
+    qr::barrier_all(ctas);
+    if (tid < j) {
+      C_ acc = cxzero<R>();
+      for (int lp = tid; lp < j; ++lp) acc = acc + T[tid][lp] * s_w[lp];
+      T[tid][j] = -(tj * acc);
+    }
+    if (tid == 0) T[j][j] = tj;
+    // Y[:, j] = tau (A[:, c+1:] v[c+1:] - Y_j w2): partial sum q % 4 a thread, sixteen loads in flight
+    const int m = n - c - 1, m4 = m & ~3, s4 = lane & 3;
+    for (int i0 = 0; i0 < rows; i0 += nt / 4) {
+      const int i = i0 + (tid >> 2);
+      const bool in = i < rows;
+      const C_* ar = A + (in ? r0 + i : r0) + (long long)(c + 1) * lda;
+      const C_* vv = sv + c + 1;
+      C_ acc = cxzero<R>();
+      int q = s4;
+      for (; q + 60 < m4; q += 64) {
+        C_ a[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) a[u] = ar[(long long)(q + 4 * u) * lda];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) acc = cxfma(a[u], vv[q + 4 * u], acc);
+      }
+      for (; q < m4; q += 4) acc = cxfma(ar[(long long)q * lda], vv[q], acc);
+      if (s4 == 0)
+        for (q = m4; q < m; ++q) acc = cxfma(ar[(long long)q * lda], vv[q], acc);
+      C_ o = cxmk<R>(__shfl_xor_sync(0xffffffffu, acc.x, 2), __shfl_xor_sync(0xffffffffu, acc.y, 2));
+      acc = acc + o;                                            // acc0 + acc2, acc1 + acc3
+      o = cxmk<R>(__shfl_xor_sync(0xffffffffu, acc.x, 1), __shfl_xor_sync(0xffffffffu, acc.y, 1));
+      C_ y = acc + o;
+      if (in && s4 == 0) {
+        for (int l = 0; l < j; ++l) y = y - sY[l * rp + i] * s_w[l];
+        y = ident ? cxzero<R>() : tj * y;
+        sY[j * rp + i] = y;
+        Y[r0 + i + (long long)j * n] = y;
+      }
+    }
+    __syncthreads();
+  }
+  // T^H, column-major kHrdPanel x kHrdPanel, for the trailing update's X = T^H W
+  if (rank == 0)
+    for (int e = tid; e < kHrdPanel * kHrdPanel; e += nt) {
+      const int r = e % kHrdPanel, cc = e / kHrdPanel;
+      TH[e] = (r < bb && cc < bb) ? cxconj(T[cc][r]) : cxzero<R>();
+    }
+  qr::barrier_all(ctas);                                        // no CTA leaves while another may still send to it
+}
+
 // --------------------------------------------- 2b. Q from the reflectors in panels (FP32 form)
 // Q = H_0 H_1 ... H_{n-3} is formed as unghr_kernel forms it, last reflectors first, but
 // kHrdPanel reflectors at a time: their product is I - V T V^H (T upper triangular, built
@@ -974,7 +1166,18 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
     const double2 one = make_double2(1.0, 0.0), mone = make_double2(-1.0, 0.0), zero = make_double2(0.0, 0.0);
     for (int k = 0; k + 2 < n; k += BB) {
       const int bb = min(BB, n - 2 - k);
-      gehrd_panel_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, k, bb, Z, z_bs); note_launch();
+      bool spread = false;
+      if constexpr (sizeof(R) == 4) {
+        int c = 1;
+        while (2 * c <= 8 && 2LL * c * batch <= sm_count()) c *= 2;
+        const size_t smc = hrd_panel_shared(n, c);
+        if (c > 1 && smc <= 200 * 1024) {
+          launch_cluster(s, gehrd_panel_cluster_kernel, c, batch, kHrdClusterThreads, smc, A, n, lda, a_bs, tau, k, bb,
+                         Z, z_bs, th);
+          spread = true;
+        }
+      }
+      if (!spread) { gehrd_panel_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, k, bb, Z, z_bs); note_launch(); }
       const int c0 = k + bb, m = n - c0, rows = n - k - 1;
       if (m <= 0) continue;
       Cx<R>* Ac = A + (long long)c0 * lda;
