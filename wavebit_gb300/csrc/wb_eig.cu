@@ -255,6 +255,28 @@ __global__ void __launch_bounds__(1024) gehrd_kernel(Cx<R>* __restrict__ Aall, i
 // matrix (column-major, ld n): V, conj(V), Y (n x kHrdPanel), W, X (kHrdPanel x n), T^H.
 constexpr int kHrdPanel = 32;
 
+// A row times v by four lanes, one a partial sum (q % 4), UN loads in flight: (s0 + s2) + (s1 + s3) in each
+// of the four. The tail past the last multiple of four belongs to the first.
+template <int UN>
+__device__ __forceinline__ Cx<float> row_times(const Cx<float>* ar, int lda, const Cx<float>* vv, int m) {
+  using C_ = Cx<float>;
+  const int m4 = m & ~3, s4 = threadIdx.x & 3;
+  C_ acc = cxzero<float>();
+  int q = s4;
+  for (; q + 4 * (UN - 1) < m4; q += 4 * UN) {
+    C_ a[UN];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) a[u] = ar[(long long)(q + 4 * u) * lda];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) acc = cxfma(a[u], vv[q + 4 * u], acc);
+  }
+  for (; q < m4; q += 4) acc = cxfma(ar[(long long)q * lda], vv[q], acc);
+  if (s4 == 0)
+    for (q = m4; q < m; ++q) acc = cxfma(ar[(long long)q * lda], vv[q], acc);
+  acc = acc + cxmk<float>(__shfl_xor_sync(0xffffffffu, acc.x, 2), __shfl_xor_sync(0xffffffffu, acc.y, 2));
+  return acc + cxmk<float>(__shfl_xor_sync(0xffffffffu, acc.x, 1), __shfl_xor_sync(0xffffffffu, acc.y, 1));
+}
+
 template <class R>
 __global__ void __launch_bounds__(1024) gehrd_panel_kernel(Cx<R>* __restrict__ Aall, int n, int lda, long long a_bs,
                                                            Cx<R>* __restrict__ tau_all, int k, int bb,
@@ -287,6 +309,7 @@ __global__ void __launch_bounds__(1024) gehrd_panel_kernel(Cx<R>* __restrict__ A
     // b = a_c - Y_j conj(V_j(c, :))
     for (int r = tid; r < n; r += nt) {
       C_ acc = A[r + (long long)c * lda];
+#pragma unroll 8
       for (int l = 0; l < j; ++l) acc = acc - Y[r + (long long)l * n] * s_vc[l];
       sb[r] = acc;
     }
@@ -309,6 +332,7 @@ __global__ void __launch_bounds__(1024) gehrd_panel_kernel(Cx<R>* __restrict__ A
       __syncthreads();
       for (int r = k + 1 + tid; r < n; r += nt) {
         C_ acc = sb[r];
+#pragma unroll 8
         for (int l = 0; l < j; ++l) acc = acc - V[r + (long long)l * n] * s_u[l];
         sb[r] = acc;
       }
@@ -363,8 +387,21 @@ __global__ void __launch_bounds__(1024) gehrd_panel_kernel(Cx<R>* __restrict__ A
     }
     if (tid == 0) T[j][j] = tj;
     __syncthreads();
-    // Y[:, j] = tau (A[:, c+1:] v[c+1:] - Y_j w2), one row per thread, four loads in flight
+    // Y[:, j] = tau (A[:, c+1:] v[c+1:] - Y_j w2): four threads a row in FP32 (eight loads in flight each: a
+    // thread a row and four loads ran on their latency), one row per thread in the other forms
     const int m = n - c - 1;
+    if constexpr (sizeof(R) == 4) {
+      for (int i0 = 0; i0 < n; i0 += nt / 4) {
+        const int r = i0 + (tid >> 2);
+        const bool in = r < n;
+        C_ y = row_times<8>(A + (in ? r : 0) + (long long)(c + 1) * lda, lda, sv + c + 1, m);
+        if (in && (tid & 3) == 0) {
+#pragma unroll 8
+          for (int l = 0; l < j; ++l) y = y - Y[r + (long long)l * n] * s_w[l];
+          Y[r + (long long)j * n] = ident ? cxzero<R>() : tj * y;
+        }
+      }
+    } else
     for (int r = tid; r < n; r += nt) {
       const C_* ar = A + r + (long long)(c + 1) * lda;
       const C_* vv = sv + c + 1;
@@ -543,30 +580,12 @@ __global__ void __launch_bounds__(kHrdClusterThreads) gehrd_panel_cluster_kernel
       T[tid][j] = -(tj * acc);
     }
     if (tid == 0) T[j][j] = tj;
-    // Y[:, j] = tau (A[:, c+1:] v[c+1:] - Y_j w2): partial sum q % 4 a thread, sixteen loads in flight
-    const int m = n - c - 1, m4 = m & ~3, s4 = lane & 3;
+    // Y[:, j] = tau (A[:, c+1:] v[c+1:] - Y_j w2), four threads a row
     for (int i0 = 0; i0 < rows; i0 += nt / 4) {
       const int i = i0 + (tid >> 2);
       const bool in = i < rows;
-      const C_* ar = A + (in ? r0 + i : r0) + (long long)(c + 1) * lda;
-      const C_* vv = sv + c + 1;
-      C_ acc = cxzero<R>();
-      int q = s4;
-      for (; q + 60 < m4; q += 64) {
-        C_ a[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) a[u] = ar[(long long)(q + 4 * u) * lda];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) acc = cxfma(a[u], vv[q + 4 * u], acc);
-      }
-      for (; q < m4; q += 4) acc = cxfma(ar[(long long)q * lda], vv[q], acc);
-      if (s4 == 0)
-        for (q = m4; q < m; ++q) acc = cxfma(ar[(long long)q * lda], vv[q], acc);
-      C_ o = cxmk<R>(__shfl_xor_sync(0xffffffffu, acc.x, 2), __shfl_xor_sync(0xffffffffu, acc.y, 2));
-      acc = acc + o;                                            // acc0 + acc2, acc1 + acc3
-      o = cxmk<R>(__shfl_xor_sync(0xffffffffu, acc.x, 1), __shfl_xor_sync(0xffffffffu, acc.y, 1));
-      C_ y = acc + o;
-      if (in && s4 == 0) {
+      C_ y = row_times<16>(A + (in ? r0 + i : r0) + (long long)(c + 1) * lda, lda, sv + c + 1, n - c - 1);
+      if (in && (tid & 3) == 0) {
         for (int l = 0; l < j; ++l) y = y - sY[l * rp + i] * s_w[l];
         y = ident ? cxzero<R>() : tj * y;
         sY[j * rp + i] = y;

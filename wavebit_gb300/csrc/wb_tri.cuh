@@ -191,11 +191,10 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_kernel(Cx<R>* __restri
       for (unsigned c = 0; c < ctas; ++c) put_remote(&sh.jrow[buf][lane], c, v);
     }
     barrier_all(ctas);
-    const int cand = (lane & (kPanelMaxCluster - 1)) % (int)ctas;
+    const int cand = lane & ((int)ctas - 1);                  // (a power of two)
     Pivot<R> top = {sh.val[buf][cand], sh.idx[buf][cand]};
-#pragma unroll
-    for (int o = kPanelMaxCluster / 2; o > 0; o >>= 1) top.meet(o, lane);
-    const int from = (top.i - k0) / rows;                     // the CTA with that row
+    for (int o = (int)ctas / 2; o > 0; o >>= 1) top.meet(o, lane);
+    const int from = ctas == 1 ? 0 : (top.i - k0) / rows;     // the CTA with that row
     // no finite candidate (NaN): the row itself, as a search that finds nothing larger
     const bool found = top.i != kNone;
     const int p = found ? top.i : gj;
