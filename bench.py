@@ -295,9 +295,9 @@ def hbm_peak():
 #: DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic byte of the QR
 #: sweep, from one small-case capture of each kernel (profiles/hseqr_*); the bench scales its live
 #: algorithmic bytes by it.
-QR_TRAFFIC_PER_ALGORITHMIC_BYTE = {'float': 643547068928 / 7.58558e11}
+QR_TRAFFIC_PER_ALGORITHMIC_BYTE = {'float': 643236118016 / 7.59664e11}
 QR_TRAFFIC_SOURCE = ('ncu dram__bytes_read.sum + dram__bytes_write.sum of one hseqr_kernel<float> launch on 4 '
-                     'solves (16 matrices, 643.5 GB against 758.6 GB algorithmic), scaled by the live '
+                     'solves (16 matrices, 643.2 GB against 759.7 GB algorithmic), scaled by the live '
                      'algorithmic bytes (profiles/hseqr_fp32_orders12_4solves.md)')
 
 
@@ -566,7 +566,7 @@ def main():
         per_launch = qr['bytes'] / qr['launches'] if qr['launches'] else None
         ratio = QR_TRAFFIC_PER_ALGORITHMIC_BYTE.get(qr['type'])
         roof = {'bound': 'hbm', 'kernel': f"wb::hseqr_kernel<{qr['type']}> (Schur-form QR sweeps, {B * L} "
-                f"matrices of {n}x{n} per launch, one CTA each)",
+                f"matrices of {n}x{n} per launch, a cluster of 1 to 8 CTAs each)",
                 'achieved': achieved, 'peak': hbm, 'unit': 'GB/s', 'frac': achieved / hbm if achieved else None,
                 'peak_source': hbm_src,
                 'algorithmic_bytes_per_launch': per_launch,
@@ -576,9 +576,9 @@ def main():
                 'traffic': per_launch * ratio if (per_launch and ratio) else None,
                 'traffic_source': QR_TRAFFIC_SOURCE if ratio else None,
                 'share_of_step': (qr['ms'] / 1e3) / t if t > 0 else None,
-                'limiter': ('the bulge step\'s barrier rather than bandwidth: ncu warp-state stalls of one launch on '
-                            '4 solves (FP32 form) give 7.2 barrier and 2.9 long-scoreboard cycles of 17.7 per issued '
-                            'instruction'),
+                'limiter': ('the latency of the chase (a reflector and the 2 x 2 core it acts on, 670 cycles a step in '
+                            'FP32, 2140 in FP64) beside the far updates\' traffic, which at one matrix per SM takes '
+                            'about as long'),
                 'whole_step': {'achieved': (280 * L + 192) * n ** 3 * B / (t / args.steps) / 1e12,
                                'unit': 'TFLOP/s', 'flops_convention': '(280 L + 192) n^3 per solve (the reference '
                                'formulation; the cascade here does about 53 n^3 per layer against its 168 n^3)'}}

@@ -275,7 +275,8 @@ long long wb_kernel_launches(wb_handle* h);
  * LAPACK and torch). */
 #define WB_TUNE_QR_THREADS 0     /* threads of a QR-sweep CTA (64..1024, multiple of 32; held to 128..512 in
                                     FP32 and 128..256 in the other forms) */
-#define WB_TUNE_HRD_THREADS 1    /* threads of a Hessenberg-reduction CTA (64..1024, multiple of 32) */
+#define WB_TUNE_HRD_THREADS 1    /* threads of a Hessenberg-reduction CTA (64..1024, multiple of 32); FP64 matrices
+                                    of 33..512 take 256 */
 #define WB_TUNE_LU_THREADS 2     /* reserved: threads of an LU / triangular-solve CTA */
 #define WB_TUNE_TENSOR_CORES 3   /* 1: complex products on the SIMT kernels instead of tcgen05 */
 #define WB_TUNE_HRD_BLOCKED 4    /* 1: the FP32 Hessenberg reduction one column at a time instead of in panels */

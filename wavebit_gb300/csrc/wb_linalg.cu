@@ -556,8 +556,9 @@ __global__ void __launch_bounds__(256) lu_update_kernel(Cx<R>* __restrict__ Aall
 
 // CTAs a matrix (a cluster) for a panel of m rows, and its shape. The panel sits in the CTAs' shared
 // memory, so C is at least what that takes. FP32: one CTA if it holds the panel, a column costs latency
-// (barriers, a reciprocal) and a cluster's barrier costs more of it: 93 -> 30 us a panel of 450 rows. FP64:
-// a row's update is FP64 issue, so up to 8 CTAs while the batch leaves SMs idle: 600 -> 100 us.
+// (barriers, a reciprocal) and a cluster's barrier costs more of it: 62 us a panel of 32 x 450 matrices (93 with
+// the rows in memory). FP64: a row's update is FP64 issue, so up to 8 CTAs while the batch leaves SMs idle:
+// 32 matrices of 242 540 -> 112 us a panel, 8 of 450 123 us, one of 50 68 us.
 struct PanelShape { int ctas, rows, threads, slices; size_t smem; };
 template <class R> static PanelShape panel_shape(int batch, int m, int kb) {
   PanelShape p;
@@ -582,7 +583,7 @@ void getrf(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a_bs, 
   st_div = st_div < 1 ? 1 : st_div;
   // One CTA a matrix: FP32 and double-float batches that fill the GPU so, and what a panel or two would
   // cover. FP64 takes the panels from the second one on, whatever the batch: its updates run on the
-  // tensor cores there, on the FP64 pipes here (n = 50: 830 -> 230 us).
+  // tensor cores there, on the FP64 pipes here (n = 50: 830 -> 230 us a factorisation).
   constexpr bool fp64 = std::is_same<R, double>::value;
   if (fp64 ? n <= LU_PB : (batch >= 2 * sm_count() || n < 2 * LU_PB)) {
     getrf_kernel<R><<<batch, LU_THREADS, 0, s>>>(A, n, lda, a_bs, ipiv, piv_bs, status, st_div);
@@ -762,7 +763,7 @@ __global__ void __launch_bounds__(256) getrs_kernel(
 
 // Few right-hand sides (the cascade's incidence columns), by a cluster a matrix (tri::getrs_narrow_kernel).
 // FP32 is bound by the diagonal blocks' chains and needs a second CTA only for its loads' sake; FP64's
-// updates are FP64 issue. 3 columns at n = 450: FP64 3.0 -> 0.4 ms, FP32 6 columns 1.0 -> 0.2 ms.
+// updates are FP64 issue. 3 columns at n = 450: FP64 3.0 -> 0.66 ms (8 matrices), FP32 6 columns 1.0 -> 0.30 ms (32).
 template <class R, int NC>
 static bool getrs_narrow(cudaStream_t s, int batch, int n, const Cx<R>* LU, int lda, long long a_bs, const int* ipiv,
                          long long piv_bs, Cx<R>* B, int nrhs, int ldb, long long b_bs) {
@@ -833,7 +834,8 @@ __global__ void __launch_bounds__(256) trans_update_kernel(const Cx<double>* __r
 // diagonal block is solved for every column (tri::trsm_diag_kernel, in FP32's upper solve
 // trsm_upper_f32_kernel) and the batched GEMM subtracts the block's contribution from the rows still to
 // solve. The substitution order and pivots are those of getrs_kernel; only the summation
-// order differs. A diagonal block of 450 columns: FP64 400 -> 80 us, FP32 65 -> 20 us.
+// order differs. A diagonal block of 450 columns: FP64 400 -> 76 us
+// (8 matrices), FP32 65 -> 39 us lower and 49 us upper (32 matrices).
 constexpr int TB_NB = tri::kTB;
 
 template <class R>

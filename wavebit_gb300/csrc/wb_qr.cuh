@@ -10,10 +10,10 @@
 // touches -- rows k, k+1 of the columns to the right, columns k, k+1 of the rows above, Z -- only
 // has to see the reflectors in order. The chain is therefore cut into windows of QrWin<R>::m
 // reflectors [k0, k1):
-//   chase   one warp runs the window's reflectors. Every lane carries the 2 x 2 core and the
+//   chase   one warp runs the window's reflectors. In FP32 every lane carries the 2 x 2 core and the
 //           reflector (no hand-over, no barrier); lane j also carries column k0 + 2 + j of the
-//           window down its rows, and the element it finishes joins the core by a shuffle. The
-//           window's columns sit in shared memory (the tile).
+//           window down its rows, and the element it finishes joins the core by a shuffle. In FP64
+//           four lanes share a pair (chase64_step). The window's columns sit in shared memory (the tile).
 //   far     the other warps apply the window before: one thread a row (of Z, and of H above the
 //           window) carries its element through the window's columns; one thread a column to the
 //           right carries it down the window's rows, through a 32-column tile in shared memory.
@@ -30,13 +30,14 @@
 // times as long. So every role is a function of its own, its state kept in shared memory between
 // windows, and a CTA has at most 512 (FP32) or 256 threads.
 //
-// What bounds it: the chase's latency. In FP32 a reflector (a square root and three divisions) and
-// the core's update take about 700 cycles a step, 1000 with the sweep's start, against 2400..4500 for
-// one barrier a reflector over the whole CTA; in FP64, where an instruction holds a scheduler for 64
-// cycles whatever its active lanes, 3600 against 11000..19000. Measured on a GB300 (one layer matrix
-// an SM or fewer): the whole mixed solve of 2 x orders (10, 9) 948 -> 400 ms, the FP64 spectrum of 16 x
-// 2 layers at orders (5, 5) 671 -> 412 ms; at n = 1250 and one matrix per SM the far updates' memory
-// traffic (2 (2n - 2) complex values a reflector) is next.
+// What bounds it: the chase's latency. In FP32 a reflector (a square root and three reciprocals, two of
+// them at once) and the core's update take 670 cycles a step, 900 with the windows' and sweeps' starts,
+// against 2400..4500 for one barrier a reflector over the whole CTA; in FP64, where an instruction holds a
+// scheduler for 64 cycles whatever its active lanes, 2140 and 2500 against 11000..19000 (some 16 FP64
+// instructions a step, each handing over to shuffles). Measured on a GB300 (one layer matrix an SM or
+// fewer): the sweep of 2 matrices of 798 in FP32 some 760 -> 215 ms, of 32 of 242 in FP64 446 -> 95 ms; at
+// n = 1250 and one matrix per SM the far updates' memory traffic (2 (2n - 2) complex values a reflector)
+// is next.
 #pragma once
 #include <type_traits>
 #include "wb_common.cuh"
@@ -92,7 +93,7 @@ __device__ __forceinline__ void right_pair(Cx<float> t1, Cx<float> v2, float t2,
   a = a - sum; b = right_sub(b, sum, cxconj(v2));
 }
 // FP64: the rotation G = [[conj(c), s], [-s, c]] with c = t1, s = t2 real: 12 operations instead of
-// 14, and no division to form it (chase_reflector). An FP64 instruction holds a scheduler for 64
+// 14, and no division to form it (chase64_step, chase_reflector). An FP64 instruction holds a scheduler for 64
 // cycles on GB300, so their number is the cost.
 __device__ __forceinline__ void left_pair(Cx<double> c, Cx<double>, double s, Cx<double>& a, Cx<double>& b) {
   const Cx<double> p = a, q = b;
