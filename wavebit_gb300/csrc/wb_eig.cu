@@ -1087,7 +1087,9 @@ template <class R> static QrShape qr_shape(int batch, int n) {
   int c = 1;
   while (2 * c <= want && 2LL * c * batch <= sms) c *= 2;
   const long long per_sm = ((long long)batch * c + sms - 1) / sms;
-  const int cap = sizeof(R) == 4 ? (per_sm <= 1 ? 16 : per_sm <= 2 ? 7 : 4) : (per_sm <= 2 ? 8 : 5);
+  // More matrices than SMs: past n = 256 a tick's far updates outlast its chase, and the largest CTA wins over
+  // several small ones (512 matrices of 450, FP32: 4 warps 784 ms, 8 656, 16 451; FP64: 5 warps 8.1 s, 8 4.2).
+  const int cap = sizeof(R) == 4 ? (per_sm <= 1 || n >= 256 ? 16 : per_sm <= 2 ? 7 : 4) : 8;
   int warps = (tasks + c - 1) / c + 1;
   warps = warps > cap ? cap : warps < 4 ? 4 : warps;
   QrShape s;

@@ -1164,7 +1164,11 @@ __global__ void __launch_bounds__(QrMaxThreads<R>::v) hseqr_kernel(Cx<R>* __rest
   {
     const int nw = blockDim.x >> 5, own = (sizeof(R) > 4 && ctas > 1) ? 0 : nw - (nw + 3) / 4 - 1, c = (int)ctas;
     nworkers = own + nw * (c - 1);
-    if (rank > 0) worker = warp < own ? warp * c + (int)rank : own * c + (warp - own) * (c - 1) + (int)rank - 1;
+    if (f64 && c == 1 && n >= 160) {                         // far updates bound a tick: the chase's scheduler too
+      nworkers = nw - 2;
+      worker = warp - 2;
+    }
+    else if (rank > 0) worker = warp < own ? warp * c + (int)rank : own * c + (warp - own) * (c - 1) + (int)rank - 1;
     else if (warp > 1 && warp % 4 != 0 && own > 0) worker = (warp - 2 - warp / 4) * c;
   }
   if (threadIdx.x == 0) {
