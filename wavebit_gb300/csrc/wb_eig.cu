@@ -723,7 +723,8 @@ __global__ void __launch_bounds__(1024) unghr_kernel(Cx<R>* __restrict__ Aall, i
 }
 
 // ---------------------------------------------------------- 3. Schur form by shifted QR: wb_qr.cuh
-// FP64 matrices of up to kQrSmall take the sweep element by element, one CTA a matrix and one
+// FP64 matrices of up to kQrSmall (and double-float batches past the GPU) take the sweep element by element, one
+// CTA a matrix and one
 // barrier a reflector: the windows of wb_qr.cuh are 16 reflectors wide and their two ticks a sweep
 // (a window, and its far updates before the next sweep) cost more there. These are the 32 x 32 group
 // blocks of the mixed form's Newton steps, thousands at a time, most of them diagonal.
@@ -1087,9 +1088,12 @@ template <class R> static QrShape qr_shape(int batch, int n) {
   int c = 1;
   while (2 * c <= want && 2LL * c * batch <= sms) c *= 2;
   const long long per_sm = ((long long)batch * c + sms - 1) / sms;
-  // More matrices than SMs: past n = 256 a tick's far updates outlast its chase, and the largest CTA wins over
-  // several small ones (512 matrices of 450, FP32: 4 warps 784 ms, 8 656, 16 451; FP64: 5 warps 8.1 s, 8 4.2).
-  const int cap = sizeof(R) == 4 ? (per_sm <= 1 || n >= 256 ? 16 : per_sm <= 2 ? 7 : 4) : 8;
+  // More matrices than SMs: small CTAs side by side, as many as the registers take (modes of 600 matrices of
+  // 242, FP32: 4 warps 231 ms, 6 206, 8 221; FP64: 4 warps 1.23 s, 5 1.59, 8 1.33), until a tick's far updates
+  // outlast its chase and the largest CTA wins (sweep of 512 of 450, FP32: 4 warps 784 ms, 8 656, 16 451;
+  // FP64: 4 warps 5.0 s, 5 8.1, 8 4.2).
+  const int cap = sizeof(R) == 4 ? (per_sm <= 1 || n >= 256 ? 16 : per_sm <= 2 ? 7 : 6)
+                                 : (per_sm <= 1 || n >= 320 ? 8 : 4);
   int warps = (tasks + c - 1) / c + 1;
   warps = warps > cap ? cap : warps < 4 ? 4 : warps;
   QrShape s;
@@ -1252,8 +1256,10 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
   }
   if (timed) cudaEventRecord(e0, s);
   bool launched = false;
-  if constexpr (std::is_same<R, double>::value) {
-    if (n <= kQrSmall) {
+  if constexpr (sizeof(R) > 4) {
+    // the element-by-element sweep: small FP64 matrices, and double-float ones that fill the GPU (the same bits;
+    // modes of 600 matrices of 50 / 126 / 242: 24 / 169 / 1080 ms against 35 / 228 / 1260 in windows)
+    if (std::is_same<R, double>::value ? n <= kQrSmall : batch > sm_count()) {
       hseqr_small_kernel<R><<<batch, 128, (size_t)n * sizeof(Cx<R>), s>>>(A, n, lda, a_bs, Z, ldz, z_bs, w, status,
                                                                          st_div < 1 ? 1 : st_div, itmax, live);
       launched = true;
