@@ -723,11 +723,10 @@ __global__ void __launch_bounds__(1024) unghr_kernel(Cx<R>* __restrict__ Aall, i
 }
 
 // ---------------------------------------------------------- 3. Schur form by shifted QR: wb_qr.cuh
-// FP64 matrices of up to kQrSmall (and double-float batches past the GPU) take the sweep element by element, one
-// CTA a matrix and one
-// barrier a reflector: the windows of wb_qr.cuh are 16 reflectors wide and their two ticks a sweep
-// (a window, and its far updates before the next sweep) cost more there. These are the 32 x 32 group
-// blocks of the mixed form's Newton steps, thousands at a time, most of them diagonal.
+// FP64 matrices of up to kQrSmall, and double-float batches past the GPU, take the sweep element by
+// element, one CTA a matrix and one barrier a reflector: the windows of wb_qr.cuh are 16 reflectors wide
+// and their two ticks a sweep (a window, and its far updates before the next sweep) cost more there. The
+// FP64 ones are the 32 x 32 group blocks of the mixed form's Newton steps, most of them diagonal.
 constexpr int kQrSmall = 32;
 
 template <class R>
