@@ -570,6 +570,7 @@ __global__ void __launch_bounds__(kNarrowThreads) getrs_narrow_kernel(const Cx<R
     const int r = e % n, c = e / n;
     X[e] = (c < nrhs) ? B[perm[r] + (long long)c * ldb] : cxzero<R>();
   }
+  barrier_all(ctas);                                          // every copy of X is filled before a solution is sent to it
   const int nblk = (n + NB - 1) / NB;
   for (int sweep = 0; sweep < 2; ++sweep) {
     const bool fwd = sweep == 0;                              // L (unit lower), then U (upper)
