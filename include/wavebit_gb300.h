@@ -42,7 +42,10 @@ extern "C" {
 #define WB_ST_GRAZING 8    /* min|w| < 1e-9 max|w|: the reference rebuilds such a layer
                               (rcwa/_engine/solve_2d.py:2463-2482); the result is flagged */
 
-#define WB_PRECISION_FP64 0        /* IEEE FP64 throughout */
+#define WB_PRECISION_FP64 0        /* FP64 throughout; its products as exact integer slices on the tensor cores,
+                                      each entry of C = A B to 2^-53 of itself plus K 2^-56 of the largest
+                                      entries of its row of A and column of B (each k balanced between the
+                                      two): WB_TUNE_TENSOR_CORES = 1 takes IEEE multiply-adds instead */
 #define WB_PRECISION_MIXED 1       /* FP32 eigen-solve brought to FP64 accuracy by Newton steps
                                       against the FP64 operator; FP32 cascade whose amplitudes are
                                       refined against the double-float interface equations */

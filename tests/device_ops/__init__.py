@@ -23,7 +23,8 @@ def load():
                         os.path.join(HERE, 'ops.cu'), '-L', PKG, '-l:libwbgpu.so', '-Xlinker', f'-rpath={PKG}'],
                        check=True, capture_output=True)
         _ops = ctypes.CDLL(out)
-        i, ll, p = ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p
+        i, ll, p, d = ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p, ctypes.c_double
         _ops.ops_getrf.argtypes = [i, i, i, p, ll, p, p]
         _ops.ops_getrs.argtypes = [i, i, i, p, ll, p, p, i, i]
+        _ops.ops_zgemm.argtypes = [i, i, i, i, d, d, p, p, p, i, p, p, i, d, d, p, p]
     return _ops

@@ -19,4 +19,18 @@ int ops_getrs(int is_double, int batch, int n, const void* LU, long long a_bs, c
   else getrs<float>(0, batch, n, (const Cx<float>*)LU, n, a_bs, piv, n, (Cx<float>*)B, nrhs, n, b_bs, trans);
   return (int)cudaGetLastError();
 }
+
+// C = (ar + i ai) op(A) op(B) + (br + i bi) C; strides in elements (rows, columns, batch). idx: A's batch index
+int ops_zgemm(int batch, int m, int n, int k, double ar, double ai, const void* A, const long long* as, const int* idx,
+              int conj_a, const void* B, const long long* bs, int conj_b, double br, double bi, void* C,
+              const long long* cs) {
+  const double2 alpha = make_double2(ar, ai), beta = make_double2(br, bi);
+  if (idx)
+    gemm_idx<double>(0, batch, m, n, k, alpha, (const Cx<double>*)A, as[0], as[1], as[2], idx, (const Cx<double>*)B,
+                     bs[0], bs[1], bs[2], beta, (Cx<double>*)C, cs[0], cs[1], cs[2]);
+  else
+    zgemm_conj(0, batch, m, n, k, alpha, (const cplx*)A, as[0], as[1], as[2], conj_a, (const cplx*)B, bs[0], bs[1],
+               bs[2], conj_b, beta, (cplx*)C, cs[0], cs[1], cs[2]);
+  return (int)cudaGetLastError();
+}
 }

@@ -52,7 +52,7 @@ bool tc_cgemm(cudaStream_t s, int batch, int m, int n, int k, double2 alpha, con
               long long a_cs, long long a_bs, const Cx<float>* B, long long b_rs, long long b_cs, long long b_bs,
               double2 beta, Cx<float>* C, long long c_rs, long long c_cs, long long c_bs);
 long long tc_errors();
-// complex FP64 products on the tensor cores by exact slices (wb_oz.cu); op(A), op(B): conjugated or
+// complex FP64 products on the tensor cores by exact slices (wb_oz.cuh); op(A), op(B): conjugated or
 // not; A of batch entry z at A + (a_idx ? a_idx[z] : z) * a_bs. False when not applicable (a
 // dimension below 8, complex alpha or beta, switched off)
 bool oz_zgemm(cudaStream_t s, int batch, int m, int n, int k, double2 alpha, const cplx* A, long long a_rs,

@@ -4,29 +4,40 @@
 // small integers exactly. C = alpha op(A) op(B) + beta C therefore runs on exact slices (the splitting
 // of Ozaki, Ogita, Oishi and Rump, "Error-free transformations of matrix multiplication", 2012, in its
 // tensor-core form of Mukunoki, Ozaki, Ogita and Imamura, 2020):
-//   - a row of A (a column of B) is scaled by the power of two of its largest entry to 63-bit fixed
-//     point, by integer operations on the doubles' bits, and cut into 8 balanced digits of 8 bits,
-//     |d| <= 128, kept as FP16;
+//   - a row of A (a column of B) is scaled by the power of two of its largest entry to fixed point, by
+//     integer operations on the doubles' bits, its largest entry in [2^61, 2^62), and cut into 8 balanced
+//     digits of 8 bits, |d| <= 128, kept as FP16;
 //   - the products of digit planes i and j with i + j = w < 8 go to one FP32 accumulator per w. K is
 //     taken 64 complex (128 real) at a time, so an accumulator holds at most 8 x 128 products of at
 //     most 2^14: integers up to 2^24, exact in FP32;
 //   - the eight accumulators are put together as integers and rounded once to FP64.
-// An entry is kept to 2^-63 of its row's (column's) largest, the dropped products (w >= 8) are below
-// 2^-64 of the largest product: a result is at least as close as a chain of FP64 FMAs unless the row's
-// entries span more than ten binary orders, and then to 2^-53 of the row's and column's norms.
+//
+// Operands graded along k (modes scaled by any factors against their inverse, the columns of U against the
+// rows of a solution) would lose what lies far below a line's largest entry, though its partner is as far
+// above: so each k of a tile's panel is first scaled by a power of two too, its column of A by 2^s and its row
+// of B by 2^-s, with s half of how much further below their lines' largest the column's entries stay
+// than the row's. The product of two lines' largest entries only falls by it. Powers of two on rows and columns
+// change no bits; on a k (against its inverse) they move the error by a binary order at most.
+//
+// Error of a panel: an entry keeps 2^-62 of its scaled line's largest, the dropped pairs (w >= 8) are below
+// 2^-57 of the two lines' largest a term, and the sum is rounded once. Where a line's entries, scaled so,
+// stay within some four binary orders, that is below a chain of FP64 FMAs' error; beyond, the error is normwise:
+// K 2^-56 of the two scaled lines' largest entries, not of each sum |a||b|. Subnormal entries and results count
+// in full. An infinity or NaN in a row or column makes that row or column of C NaN.
 //
 // A complex product is one real product of twice the size, [Re -Im; Im Re] [Re; Im], so a CTA's 64 x 64
 // complex tile is one 128 x 64 accumulator for each of 8 weights: all 512 columns of tensor memory.
 //
-// Per CTA (8 warps and a ninth that issues the MMAs): a pass over the K panel finds the exponents;
-// then, 16 complex k at a time, warps 0..3 split A and warps 4..7 split B into the canonical no-swizzle
+// Per CTA (8 warps and a ninth that issues the MMAs): a pass over the K panel finds the scales; then, 16
+// complex k at a time, warps 0..3 split A and warps 4..7 split B into the canonical no-swizzle
 // K-major layout (two stages of 96 KB) while the MMAs of the chunk before run (36 pairs, 72 MMAs a
-// chunk). An infinity or NaN in a row or column makes that row or column of C NaN.
+// chunk).
 //
 // What bounds it: a tile's own latencies. One CTA an SM (192 KB, all of tensor memory) takes about 17 us a
-// tile of K = 64: the exponents' pass, the splitting and the 288 MMAs (5 us alone), the eight accumulators'
-// assembly, and C read and written; FP64 FMAs take 270 us. 450 x 450 x 64, 8 matrices: 107 us (7.8 TFLOP/s),
-// x 450 679 us (8.6). Holding C's entries during the MMAs spills at 168 registers and was 10% slower.
+// tile of K = 64: the scales' pass, the splitting and the 288 MMAs (5 us alone), the eight accumulators'
+// assembly, and C read and written; FP64 FMAs take 270 us. 450 x 450 x 64, 8 matrices, C read and written: 128 us
+// (6.5 TFLOP/s), 121 without the k's scales; x 450 769 us (7.6), 713 without; K = 31 the same with and without.
+// Holding C's entries during the MMAs spills at 168 registers and was 10% slower.
 // Every mbarrier wait is bounded, as in wb_tc.cuh.
 #pragma once
 #include "wb_tc.cuh"
@@ -57,14 +68,29 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_
       "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(acc));
 }
 
-// x in 63-bit fixed point for the biased exponent eb of its row's largest entry, every byte biased by
-// 128: byte 7 - i is digit i + 128
+// Exponents of lines and entries are kept with this added (0: none); kBad: an infinity or NaN in the line.
+constexpr int kOff = 4096, kBad = 1 << 20;
+// the shift of a k that contributes nothing (its column of A or row of B is zero)
+constexpr int kDropped = -30000;
+
+// The exponent of a complex entry's larger component, biased, + kSub so that subnormals' (by their leading bit,
+// down to -51) stay positive; 0 for zero.
+constexpr int kSub = 64;
+__device__ __forceinline__ int entry_exponent(double2 v) {
+  const int hx = __double2hiint(v.x) & 0x7fffffff, hy = __double2hiint(v.y) & 0x7fffffff;
+  const int e = max(hx, hy) >> 20;
+  if (e) return e + kSub;
+  const uint64_t b = ((uint64_t)(uint32_t)(hx | hy) << 32) | (uint32_t)(__double2loint(v.x) | __double2loint(v.y));
+  return b ? kSub + 12 - __clzll((long long)b) : 0;
+}
+
+// x in fixed point for the biased exponent eb of its line's largest entry (x not scaled: eb less the k's
+// shift), every byte biased by 128: byte 7 - i is digit i + 128
 __device__ __forceinline__ uint64_t fixed_bytes(double x, int eb) {
-  const int hi = __double2hiint(x);
-  const int e = (hi >> 20) & 0x7ff;
-  uint64_t m = ((uint64_t)((hi & 0xfffff) | 0x100000) << 32) | (uint32_t)__double2loint(x);
-  const int sh = e - eb + 9;
-  if (e == 0 || sh < -54) m = 0;
+  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+  uint64_t m = ((uint64_t)((hi & 0xfffff) | (min(e, 1) << 20)) << 32) | (uint32_t)__double2loint(x);
+  const int sh = max(e, 1) - eb + 9;
+  if (sh < -54) m = 0;
   else if (sh >= 0) m <<= sh;
   else m = (m + (1ull << (-sh - 1))) >> -sh;
   const uint64_t q = hi < 0 ? 0ull - m : m;
@@ -84,6 +110,16 @@ __device__ __forceinline__ uint4 halves(const uint32_t* w, int b) {
 }
 __device__ __forceinline__ uint4 negated(uint4 v) {
   return make_uint4(v.x ^ 0x80008000u, v.y ^ 0x80008000u, v.z ^ 0x80008000u, v.w ^ 0x80008000u);
+}
+
+// m (its top bit set) of biased exponent e where that is no normal number's: subnormal, or infinite
+__device__ __noinline__ double range_end(uint64_t m, int e, bool neg) {
+  uint64_t bits = 0x7ffull << 52;
+  if (e < 1) {
+    const int drop = 12 - e;
+    bits = drop > 64 ? 0 : (drop < 64 ? m >> drop : 0) + ((m >> (drop - 1)) & 1);
+  }
+  return __longlong_as_double((long long)(((uint64_t)neg << 63) | bits));
 }
 
 // sum over w of a[w] 256^(7 - w), times 2^(ea + eb) (biased exponents of the row and the column)
@@ -109,10 +145,9 @@ __device__ __forceinline__ double assemble(const float* a, int ea, int eb) {
   m |= n >= 32 ? (uint64_t)lo << (n - 32) : (uint64_t)lo >> (32 - n);
   int e = ea + eb - n - 994 - shift;
   uint64_t r = (m >> 11) + ((m >> 10) & 1);                    // 53 bits, rounded
-  if (r >> 53) { r >>= 1; ++e; }
-  if (e <= 0) return 0.0;
-  if (e >= 2047) return neg ? -INFINITY : INFINITY;
-  const uint64_t bits = ((uint64_t)neg << 63) | ((uint64_t)e << 52) | (r & 0xfffffffffffffull);
+  const int up = (int)(r >> 53);
+  if ((unsigned)(e + up - 1) >= 2046u) return range_end(m, e, neg);
+  const uint64_t bits = ((uint64_t)neg << 63) | ((uint64_t)(e + up) << 52) | ((r >> up) & 0xfffffffffffffull);
   return __longlong_as_double((long long)bits);
 }
 
@@ -132,7 +167,11 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t bars[2];
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_fail, s_exp[2 * kT];
+  __shared__ int s_fail;
+  __shared__ int s_top[2 * kT], s_line[2 * kT];                // the lines' exponents before and after the k's shifts
+  __shared__ int s_k[2 * kT];                                  // a k's largest entry, against its line's largest
+  __shared__ __align__(16) short s_shift[2 * kT];              // its shift
+  __shared__ __align__(16) short s_half[2 * kT];               // the same, even k before odd ones
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool issuer = warp == 8;
   const int row0 = blockIdx.x * kT, col0 = blockIdx.y * kT;
@@ -160,6 +199,7 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
   const long long ls = onB ? g.b_cs : g.a_rs, ks = onB ? g.b_rs : g.a_cs;
   const bool live = !issuer && (onB ? col0 + line < g.n : row0 + line < g.m);
   const double2* src = onB ? B + (long long)(col0 + line) * ls : A + (long long)(row0 + line) * ls;
+  const int side = onB ? kT : 0;
   const bool flip = (onB ? g.conj_b : g.conj_a) != 0;
 
   // an accumulator row (real or imaginary part of a complex row) and 32 columns a thread
@@ -171,22 +211,97 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
   uint32_t uses = 0;                    // chunks staged so far: buffer uses & 1, its use uses >> 1
   bool ok = true;
   for (int p0 = 0; p0 < g.k && ok; p0 += kKp) {
-    const int kk = min(kKp, g.k - p0);
-    // the lines' largest exponents over the panel (each half of a line by one thread, then the max)
-    if (tid < 2 * kT) s_exp[tid] = 0;
+    const int kk = min(kKp, g.k - p0), nchunk = (kk + kKc - 1) / kKc;
+    // the panel's scales: the lines' largest entries, the k's shifts, the lines' largest with them
+    if (tid < 2 * kT) s_top[tid] = s_line[tid] = s_k[tid] = 0;
     __syncthreads();
-    int mx = 0;
-    if (live)
-      for (int q = part; q < kk; q += 2) {
-        const double2 v = src[(p0 + q) * ks];
-        mx = max(mx, max(__double2hiint(v.x) & 0x7ff00000, __double2hiint(v.y) & 0x7ff00000));
+    // this thread's 32 exponents, two a word, in the stages' memory (their last readers were waited for)
+    uint32_t* ex = reinterpret_cast<uint32_t*>(smem) + tid;
+    const int tk = kk > 32 ? 32 : 16;
+    int top = 0;
+    bool bad = false;
+    if (!issuer) {
+      // (q = part, part + 2, ..: the two halves of a line read its sectors together)
+#pragma unroll 1
+      for (int t = 0; t < tk; t += 4) {
+        double2 w[4];
+        uint32_t e[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int q = part + 2 * (t + u);
+          w[u] = make_double2(0.0, 0.0);
+          if (live && q < kk) w[u] = src[(p0 + q) * ks];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          int x = entry_exponent(w[u]);
+          if (x == 0x7ff + kSub) { bad = true; x = 0; }
+          top = max(top, x);
+          e[u] = (uint32_t)x;
+        }
+        ex[kWorkers * (t / 2)] = e[0] | e[1] << 16;
+        ex[kWorkers * (t / 2 + 1)] = e[2] | e[3] << 16;
       }
-    if (mx) atomicMax(&s_exp[(onB ? kT : 0) + line], mx >> 20);
+      if (top) atomicMax(&s_top[side + line], top);
+    }
     __syncthreads();
-    const int eb = issuer ? 0 : s_exp[(onB ? kT : 0) + line];
-    const int nchunk = (kk + kKc - 1) / kKc;
+    if (!issuer) {
+      // the largest of the warp's 32 lines for each of its k, 16 at a time: pairs of 16 bits, halved from lane to
+      // lane until a lane holds one pair
+      const uint32_t base = (uint32_t)(kOff - s_top[side + line]);
+#pragma unroll 1
+      for (int t0 = 0; t0 < tk; t0 += 16) {
+        uint32_t w[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          const uint32_t e = ex[kWorkers * (t0 / 2 + t)];
+          w[t] = ((e & 0xffffu) ? (e & 0xffffu) + base : 0u) | ((e >> 16) ? ((e >> 16) + base) << 16 : 0u);
+        }
+#pragma unroll
+        for (int h = 4, bit = 1; h >= 1; h >>= 1, bit <<= 1)
+#pragma unroll
+          for (int t = 0; t < h; ++t) {
+            const bool up = lane & bit;
+            const uint32_t give = up ? w[t] : w[t + h], keep = up ? w[t + h] : w[t];
+            w[t] = __vmaxu2(keep, __shfl_xor_sync(0xffffffffu, give, bit));
+          }
+        w[0] = __vmaxu2(w[0], __shfl_xor_sync(0xffffffffu, w[0], 8));
+        w[0] = __vmaxu2(w[0], __shfl_xor_sync(0xffffffffu, w[0], 16));
+        const int t = t0 + (((lane & 1) << 3) | ((lane & 2) << 1) | ((lane & 4) >> 1) | (lane >> 4));
+        const int m = (int)(lane >> 4 ? w[0] >> 16 : w[0] & 0xffffu);
+        if (m && !(lane & 8)) atomicMax(&s_k[side + part + 2 * t], m);
+      }
+    }
+    __syncthreads();
+    if (tid < kT) {
+      const int a = s_k[tid], b = s_k[kT + tid], h = (b - a) >> 1;
+      const int at = (tid & 1) * 32 + (tid >> 1);
+      s_shift[tid] = s_half[at] = (short)(a && b ? h : kDropped);
+      s_shift[kT + tid] = s_half[kT + at] = (short)(a && b ? -h : kDropped);
+    }
+    __syncthreads();
+    if (!issuer) {
+      int mx = kDropped;
+#pragma unroll 1
+      for (int t = 0; t < tk; t += 8) {
+        const uint4 sv = *reinterpret_cast<const uint4*>(s_half + side + part * 32 + t);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t e = ex[kWorkers * (t / 2 + u)], h = u == 0 ? sv.x : u == 1 ? sv.y : u == 2 ? sv.z : sv.w;
+          if (e & 0xffffu) mx = max(mx, (int)(e & 0xffffu) + (short)h);
+          if (e >> 16) mx = max(mx, (int)(e >> 16) + ((int)h >> 16));
+        }
+      }
+      mx += kOff - kSub;
+      if (bad) mx = kBad;
+      if (mx > 0) atomicMax(&s_line[side + line], mx);
+    }
+    __syncthreads();
+    const int eb = issuer ? 0 : s_line[side + line] - kOff;
     double2 v[8];
+    uint4 shift;                                               // of the 8 k, 16 bits each
     auto load = [&](int c) {
+      shift = *reinterpret_cast<const uint4*>(s_shift + side + c * kKc + part * 8);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int q = c * kKc + part * 8 + u;
@@ -204,7 +319,9 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
         uint32_t rh[8], rl[8], ih[8], il[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          const uint64_t a = fixed_bytes(v[u].x, eb), b = fixed_bytes(flip ? -v[u].y : v[u].y, eb);
+          const uint32_t h = u < 2 ? shift.x : u < 4 ? shift.y : u < 6 ? shift.z : shift.w;
+          const int ek = eb - ((u & 1) ? (int)h >> 16 : (int)(short)h);
+          const uint64_t a = fixed_bytes(v[u].x, ek), b = fixed_bytes(flip ? -v[u].y : v[u].y, ek);
           rh[u] = (uint32_t)(a >> 32); rl[u] = (uint32_t)a;
           ih[u] = (uint32_t)(b >> 32); il[u] = (uint32_t)b;
         }
@@ -262,7 +379,7 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
     if (s_fail) { ok = false; break; }
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (!issuer) {
-      const int ea = s_exp[arow & 63];
+      const int ea = s_line[arow & 63];
 #pragma unroll
       for (int c8 = 0; c8 < 32; c8 += 4) {
         float t[kDig][4];
@@ -282,10 +399,10 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
           float a8[kDig];
 #pragma unroll
           for (int w = 0; w < kDig; ++w) a8[w] = t[w][j];
-          const int ec = s_exp[kT + acol0 + c8 + j];
+          const int ec = s_line[kT + acol0 + c8 + j];
           double x = 0.0;
-          if (ea == 2047 || ec == 2047) x = NAN;
-          else if (ea && ec) x = assemble(a8, ea, ec);
+          if (ea == kBad || ec == kBad) x = NAN;
+          else if (ea && ec) x = assemble(a8, ea - kOff, ec - kOff);
           acc[c8 + j] = p0 == 0 ? x : acc[c8 + j] + x;
         }
       }

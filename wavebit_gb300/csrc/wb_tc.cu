@@ -25,7 +25,7 @@ bool tc_cgemm(cudaStream_t s, int batch, int m, int n, int k, double2 alpha, con
 }
 
 // The exact-slice product serves any strides, real alpha and beta and conjugated operands. Its cost is
-// flat (about 10 us a 64 x 64 tile and 64 of K, an FP64 tile of that size 270 us), so only the thinnest
+// flat (about 17 us a 64 x 64 tile and 64 of K, an FP64 tile of that size 270 us), so only the thinnest
 // products stay on the FP64 pipes: a dimension under 8 (the right-hand-side blocks of gemm_narrow_kernel).
 bool oz_zgemm(cudaStream_t s, int batch, int m, int n, int k, double2 alpha, const cplx* A, long long a_rs,
               long long a_cs, long long a_bs, const int* a_idx, bool conj_a, const cplx* B, long long b_rs,
