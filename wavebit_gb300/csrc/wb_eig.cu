@@ -1117,10 +1117,11 @@ int hrd_threads(int batch, int n) {
   return t;
 }
 
-// Launches kernel with `ctas` CTAs a matrix as one cluster.
+// Launches kernel with `ctas` CTAs a matrix as one cluster; `most`: its largest dynamic shared memory.
 template <class... P, class... Q>
-static void launch_cluster(cudaStream_t s, void (*kernel)(P...), int ctas, int batch, int threads, size_t smem, Q... args) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static void launch_cluster(cudaStream_t s, void (*kernel)(P...), int most, int ctas, int batch, int threads, size_t smem,
+                           Q... args) {
+  allow_shared(kernel, most);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(batch * ctas));
   cfg.blockDim = dim3((unsigned)threads);
@@ -1140,13 +1141,14 @@ static void launch_cluster(cudaStream_t s, void (*kernel)(P...), int ctas, int b
 static bool reduce64(cudaStream_t s, int batch, int n, Cx<double>* A, int lda, long long a_bs, Cx<double>* Z, int ldz,
                      long long z_bs, Cx<double>* tau) {
   const size_t smem = hrd::shared_elements(n) * sizeof(Cx<double>);
-  if (n > 512 || smem > 200 * 1024) return false;
+  constexpr int most = 200 * 1024;
+  if (n > 512 || smem > most) return false;
   const int sms = sm_count();
   int c = 1;
   while (2 * c <= hrd::kParts && 2LL * c * batch <= sms) c *= 2;
-  if (n <= 64) launch_cluster(s, hrd::gehrd64_kernel<2>, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
-  else if (n <= 128) launch_cluster(s, hrd::gehrd64_kernel<4>, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
-  else launch_cluster(s, hrd::gehrd64_kernel<8>, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
+  if (n <= 64) launch_cluster(s, hrd::gehrd64_kernel<2>, most, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
+  else if (n <= 128) launch_cluster(s, hrd::gehrd64_kernel<4>, most, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
+  else launch_cluster(s, hrd::gehrd64_kernel<8>, most, c, batch, hrd::kThreads, smem, A, n, lda, a_bs, tau);
   const int groups = n <= 256 ? (n + 1) / 2 : n;
   const unsigned gx = (unsigned)max(1LL, min((long long)(groups + 3) / 4, (2LL * sms + batch - 1) / batch));
   const dim3 grid(gx, (unsigned)batch);
@@ -1166,8 +1168,8 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
                 const int* live) {
   if (batch <= 0 || n <= 0) return;
   size_t sm = 2 * (size_t)n * sizeof(Cx<R>);
-  cudaFuncSetAttribute(gehrd_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  cudaFuncSetAttribute(unghr_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  allow_shared(gehrd_kernel<R>, kVectorShared);
+  allow_shared(unghr_kernel<R>, kVectorShared);
   const int th = hrd_threads(batch, n);
   // the FP32 form at n >= 192 reduces in panels (Z, not yet formed, holds the panels' scratch:
   // 5 n kHrdPanel + kHrdPanel^2 elements, within n * ldz from n = 161 on)
@@ -1178,7 +1180,7 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
   }
   if (reduced) {
   } else if (blocked) {
-    cudaFuncSetAttribute(gehrd_panel_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    allow_shared(gehrd_panel_kernel<R>, kVectorShared / 2);
     const int BB = kHrdPanel;
     const long long nB = (long long)n * BB;
     Cx<R>* V = Z;
@@ -1195,8 +1197,9 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
         int c = 1;
         while (2 * c <= 8 && 2LL * c * batch <= sm_count()) c *= 2;
         const size_t smc = hrd_panel_shared(n, c);
-        if (c > 1 && smc <= 200 * 1024) {
-          launch_cluster(s, gehrd_panel_cluster_kernel, c, batch, kHrdClusterThreads, smc, A, n, lda, a_bs, tau, k, bb,
+        constexpr int most = 200 * 1024;
+        if (c > 1 && smc <= most) {
+          launch_cluster(s, gehrd_panel_cluster_kernel, most, c, batch, kHrdClusterThreads, smc, A, n, lda, a_bs, tau, k, bb,
                          Z, z_bs, th);
           spread = true;
         }
@@ -1259,6 +1262,7 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
     // the element-by-element sweep: small FP64 matrices, and double-float ones that fill the GPU (the same bits;
     // modes of 600 matrices of 50 / 126 / 242: 24 / 169 / 1080 ms against 35 / 228 / 1260 in windows)
     if (std::is_same<R, double>::value ? n <= kQrSmall : batch > sm_count()) {
+      allow_shared(hseqr_small_kernel<R>, kVectorShared / 2);
       hseqr_small_kernel<R><<<batch, 128, (size_t)n * sizeof(Cx<R>), s>>>(A, n, lda, a_bs, Z, ldz, z_bs, w, status,
                                                                          st_div < 1 ? 1 : st_div, itmax, live);
       launched = true;
@@ -1266,7 +1270,7 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
   }
   if (launched) note_launch();
   else
-    launch_cluster(s, hseqr_kernel<R>, shape.ctas, batch, shape.threads, shape.smem, A, n, lda, a_bs, Z, ldz, z_bs, w,
+    launch_cluster(s, hseqr_kernel<R>, kVectorShared, shape.ctas, batch, shape.threads, shape.smem, A, n, lda, a_bs, Z, ldz, z_bs, w,
                    status, st_div < 1 ? 1 : st_div, itmax);
   if (timed) cudaEventRecord(e1, s);
 }

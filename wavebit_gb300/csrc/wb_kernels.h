@@ -16,6 +16,14 @@ enum TuneKey { kTuneQrThreads = 0, kTuneHrdThreads = 1, kTuneLuThreads = 2, kTun
                kTuneKeys = 8 };
 int tuning(int key);
 void set_tuning(int key, int value);
+// The most dynamic shared memory `kernel` is launched with. The limit belongs to the function, not to a call: it is
+// a constant of the kernel, whatever the call at hand takes, so that host threads with calls of their own cannot
+// lower it between one another's setting and launch. (Static and dynamic memory: 227 KB a CTA.)
+template <class... P> inline cudaError_t allow_shared(void (*kernel)(P...), int bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+// vectors of n = 2N <= 6456 complex values: two of 16 bytes a value
+constexpr int kVectorShared = 2 * 6456 * 16;
 // multiprocessor count of the current device (cached per device)
 int sm_count();
 // live timing of the QR-sweep launches (wb_eig.cu): on/off (clears), and per real type
@@ -103,8 +111,8 @@ void normalize_columns(cudaStream_t s, int batch, int n, Cx<R>* W, int ldw, long
 // ---- order windows
 // The largest windows the kernels hold on chip: stage A inverts an (2hv+1)^2 Toeplitz matrix
 // beside its identity in one block's shared memory (32 (2hv+1)^2 bytes <= 227 KB: hv <= 42), and
-// the eigen-solve keeps vectors of n = 2N complex values in shared memory (36 n bytes for the
-// mixed form's group step: N <= 3228).
+// the eigen-solve keeps vectors of n = 2N complex values in shared memory (32 n bytes in the
+// Hessenberg reduction: kVectorShared, N <= 3228).
 inline bool orders_fit(int hu, int hv) {
   return hu >= 0 && hv >= 0 && hv <= 42 && hu <= 1613 && (2LL * hu + 1) * (2LL * hv + 1) <= 3228;
 }

@@ -594,7 +594,7 @@ void getrf(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a_bs, 
   // FP64: equal panels, so that no product is a few rows deep or wide and falls off the tensor cores
   if (fp64) { const int panels = (n + LU_PB - 1) / LU_PB; width = (n + panels - 1) / panels; }
   while (width > 8 && panel_shape<R>(batch, n, width).smem > 212 * 1024) width /= 2;
-  cudaFuncSetAttribute(tri::lu_panel_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 212 * 1024);
+  allow_shared(tri::lu_panel_kernel<R>, 212 * 1024);
   for (int k0 = 0; k0 < n; k0 += width) {
     const int kb = min(width, n - k0);
     const PanelShape sh = panel_shape<R>(batch, n - k0, kb);
@@ -773,7 +773,7 @@ static bool getrs_narrow(cudaStream_t s, int batch, int n, const Cx<R>* LU, int 
                                                   : (n < 480 ? 1 : n < 960 ? 2 : 4);
   int c = 1;
   while (2 * c <= want && 2LL * c * batch <= sm_count()) c *= 2;
-  cudaFuncSetAttribute(tri::getrs_narrow_kernel<R, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  allow_shared(tri::getrs_narrow_kernel<R, NC>, 180 * 1024);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(batch * c));
   cfg.blockDim = dim3((unsigned)(n <= 128 ? 256 : tri::kNarrowThreads));
@@ -845,12 +845,12 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
   const size_t smp = (size_t)n * (sizeof(Cx<R>) + 2 * sizeof(int));
   const int cols = max(1, (int)((long long)nrhs * batch / (4LL * sm_count())));
   const dim3 gs((nrhs + cols - 1) / cols, batch);
-  cudaFuncSetAttribute(tri::laswp_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smp);
+  allow_shared(tri::laswp_kernel<R>, kVectorShared);
   if (trans == 0) {
     tri::laswp_kernel<R><<<gs, 256, smp, s>>>(B, n, nrhs, ldb, b_bs, ipiv, piv_bs, 1, cols);
     note_launch();
   }
-  const size_t sm = sizeof(Cx<R>) * (size_t)TB_NB * (TB_NB + 1);
+  constexpr int sm = sizeof(Cx<R>) * TB_NB * (TB_NB + 1);
   // threads a column: FP32 is bound by the block's chain of shuffles; FP64 by the instructions of a warp
   // times the warps a scheduler gets
   int T = 8;
@@ -865,13 +865,13 @@ static void getrs_blocked(cudaStream_t s, int batch, int n, const Cx<R>* LU, int
     if (T == 16) kernel = tri::trsm_diag_kernel<R, 16>;
     if (T == 32) kernel = tri::trsm_diag_kernel<R, 32>;
   }
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  allow_shared(kernel, sm);
   const dim3 gd((nrhs + tri::kTriThreads / T - 1) / (tri::kTriThreads / T), batch);
   auto diagonal = [&](int i0, int ib, int lower, int unit) {
     if constexpr (sizeof(R) == 4) {
       if (!lower) {
-        const size_t su = sizeof(Cx<R>) * (size_t)(TB_NB + 32) * (TB_NB + 1);
-        cudaFuncSetAttribute(tri::trsm_upper_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su);
+        constexpr int su = sizeof(Cx<R>) * (TB_NB + 32) * (TB_NB + 1);
+        allow_shared(tri::trsm_upper_f32_kernel, su);
         tri::trsm_upper_f32_kernel<<<dim3((nrhs + 31) / 32, batch), 32, su, s>>>(
             (const Cx<float>*)LU, lda, a_bs, (Cx<float>*)B, nrhs, ldb, b_bs, i0, ib, unit, trans);
         note_launch();

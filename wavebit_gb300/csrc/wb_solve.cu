@@ -1143,7 +1143,7 @@ void stage_b_newton(cudaStream_t s, int P, int N, const cplx* conv, const int* p
   const size_t gsm = (size_t)n * 4 * sizeof(int);
   const GroupScratch gs = {(cplx*)Tm, (int*)Um, Nn};             // T and U are free between the residual and the next product
   const dim3 gcols((unsigned)max(1LL, min((long long)(n + 7) / 8, (16LL * sm_count() + P - 1) / P)), (unsigned)P);
-  cudaFuncSetAttribute(group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm);
+  allow_shared(group_kernel, kVectorShared / 2);
   for (int it = 0; it < kNewtonSteps; ++it) {
     if (it > 0) convert<double, float>(s, (const Cx<double>*)Wd, nb.F1, tot);
     cudaMemcpyAsync(nb.F2, nb.F1, sizeof(F) * tot, cudaMemcpyDeviceToDevice, s);   // W in FP32 for W E

@@ -11,7 +11,7 @@ bool tc_cgemm(cudaStream_t s, int batch, int m, int n, int k, double2 alpha, con
               double2 beta, Cx<float>* C, long long c_rs, long long c_cs, long long c_bs) {
   if (tuning(kTuneTensorCores) == 1) return false;          // switched off
   if (batch <= 0 || m < tc::kTileM || n < 64 || k < tc::kKb) return false;   // small: the SIMT kernel
-  if (cudaFuncSetAttribute(tc::cgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::kSmemBytes) !=
+  if (allow_shared(tc::cgemm_kernel, (int)tc::kSmemBytes) !=
       cudaSuccess) {
     cudaGetLastError();
     return false;
@@ -33,7 +33,7 @@ bool oz_zgemm(cudaStream_t s, int batch, int m, int n, int k, double2 alpha, con
               long long c_bs) {
   if (tuning(kTuneTensorCores) == 1) return false;          // switched off
   if (alpha.y != 0.0 || beta.y != 0.0 || m < 8 || n < 8 || k < 8) return false;
-  if (cudaFuncSetAttribute(oz::zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz::kSmem) !=
+  if (allow_shared(oz::zgemm_kernel, (int)oz::kSmem) !=
       cudaSuccess) {
     cudaGetLastError();
     return false;
