@@ -27,4 +27,5 @@ def load():
         _ops.ops_getrf.argtypes = [i, i, i, p, ll, p, p]
         _ops.ops_getrs.argtypes = [i, i, i, p, ll, p, p, i, i]
         _ops.ops_zgemm.argtypes = [i, i, i, i, d, d, p, p, p, i, p, p, i, d, d, p, p]
+        _ops.ops_schur.argtypes = [i, i, p, p, p, p, p]
     return _ops

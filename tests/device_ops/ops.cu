@@ -20,6 +20,13 @@ int ops_getrs(int is_double, int batch, int n, const void* LU, long long a_bs, c
   return (int)cudaGetLastError();
 }
 
+// Schur form: A (n x n, by columns) becomes T, Z its vectors, w its eigenvalues
+int ops_schur(int batch, int n, void* A, void* Z, void* w, void* tau, int* status) {
+  geev_schur<double>(0, batch, n, (Cx<double>*)A, n, (long long)n * n, (Cx<double>*)Z, n, (long long)n * n,
+                     (Cx<double>*)w, (Cx<double>*)tau, status, 1);
+  return (int)cudaGetLastError();
+}
+
 // C = (ar + i ai) op(A) op(B) + (br + i bi) C; strides in elements (rows, columns, batch). idx: A's batch index
 int ops_zgemm(int batch, int m, int n, int k, double ar, double ai, const void* A, const long long* as, const int* idx,
               int conj_a, const void* B, const long long* bs, int conj_b, double br, double bi, void* C,

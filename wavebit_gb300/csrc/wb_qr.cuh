@@ -921,9 +921,14 @@ __device__ __noinline__ bool near_columns64(Cx<double>* H, int ldh, Cx<double>* 
 // A subdiagonal below one unit of roundoff of its neighbours' diagonal deflates if the refined test
 // agrees (Ahues and Tisseur). Where both diagonal entries are the same number (equal eigenvalues of a
 // uniform layer, split by rounding alone) that test never does, and when the shift rounds to them too
-// a sweep only swaps the two: after 10 sweeps the FP64 form lets the first test decide.
+// a sweep only swaps the two: after 10 sweeps the FP64 form also deflates a pair that cannot be told apart, its
+// diagonal entries within tol = one unit of roundoff of their sum and its split, the root of the two off-diagonal
+// entries' product, below tol too. Any other block keeps the refined test, however slow.
 template <class R> struct QrStall { static constexpr int its = 1 << 30; };
 template <> struct QrStall<double> { static constexpr int its = 10; };
+template <class R> __device__ __forceinline__ bool same_pair(Cx<R> dd, Cx<R> sub, Cx<R> sup, R tol) {
+  return cxabs1(dd) <= tol && cxabs1(sub) * cxabs1(sup) <= tol * tol;
+}
 
 // What the chase does next, decided by the chasing warp: continue the sweep, or find the active
 // block of the next one (deflating converged eigenvalues into w), its shift and first reflector.
@@ -988,7 +993,8 @@ __device__ __noinline__ int next_window(Cx<R>* H, int n, int ldh, Cx<R>* w, int 
               R aa = rmax(cxabs1(hd), cxabs1(dd));
               R bb = rmin(cxabs1(hd), cxabs1(dd));
               R sx = aa + ab;
-              if (its >= QrStall<R>::its || ba * (ab / sx) <= rmax(smlnum, ulp * (bb * (aa / sx)))) small = true;
+              if (ba * (ab / sx) <= rmax(smlnum, ulp * (bb * (aa / sx)))) small = true;
+              else if (its >= QrStall<R>::its && same_pair<R>(dd, sub, hu, ulp * tst)) small = true;
             }
           }
         }
