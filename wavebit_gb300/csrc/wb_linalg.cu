@@ -767,13 +767,15 @@ __global__ void __launch_bounds__(256) getrs_kernel(
 template <class R, int NC>
 static bool getrs_narrow(cudaStream_t s, int batch, int n, const Cx<R>* LU, int lda, long long a_bs, const int* ipiv,
                          long long piv_bs, Cx<R>* B, int nrhs, int ldb, long long b_bs) {
-  const size_t sm = (size_t)n * (NC * sizeof(Cx<R>) + 2 * sizeof(int));
-  if (sm > (size_t)180 * 1024) return false;
+  // X in up to 200 KB (n <= 4266 at 48 bytes a row) and the permutation, beside the 17 KB of a diagonal block
+  constexpr int most_x = 200 * 1024, most = most_x + 2 * 4266;
+  const size_t x = (size_t)n * NC * sizeof(Cx<R>), sm = x + n * sizeof(unsigned short);
+  if (x > most_x) return false;
   const int want = std::is_same<R, double>::value ? (n < 64 ? 1 : n < 128 ? 2 : n < 256 ? 4 : 8)
                                                   : (n < 480 ? 1 : n < 960 ? 2 : 4);
   int c = 1;
   while (2 * c <= want && 2LL * c * batch <= sm_count()) c *= 2;
-  allow_shared(tri::getrs_narrow_kernel<R, NC>, 180 * 1024);
+  allow_shared(tri::getrs_narrow_kernel<R, NC>, most);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(batch * c));
   cfg.blockDim = dim3((unsigned)(n <= 128 ? 256 : tri::kNarrowThreads));

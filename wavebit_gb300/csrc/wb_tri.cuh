@@ -549,9 +549,9 @@ __global__ void __launch_bounds__(kNarrowThreads) getrs_narrow_kernel(const Cx<R
   constexpr int NB = 32, CG = std::is_same<R, double>::value ? 1 : NC, G = NC / CG, U = sizeof(R) == 4 ? 32 : 16;
   extern __shared__ __align__(16) unsigned char smraw[];
   C_* X = reinterpret_cast<C_*>(smraw);                       // [column][row]
-  int* perm = reinterpret_cast<int*>(X + (size_t)n * NC);
-  int* piv = perm + n;
-  __shared__ C_ sD[2][NB][NB + 1];                            // [t][r]
+  unsigned short* perm = reinterpret_cast<unsigned short*>(X + (size_t)n * NC);
+  int* piv = reinterpret_cast<int*>(X);                       // until the fill
+  __shared__ C_ sD[NB][NB + 1];                               // [t][r]
   unsigned rank, ctas;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
@@ -560,11 +560,12 @@ __global__ void __launch_bounds__(kNarrowThreads) getrs_narrow_kernel(const Cx<R
   const int* ipiv = ipiv_all + (long long)mat * piv_bs;
   C_* B = Ball + mat * b_bs;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
-  for (int i = tid; i < n; i += nt) { perm[i] = i; piv[i] = ipiv[i]; }
+  for (int i = tid; i < n; i += nt) { perm[i] = (unsigned short)i; piv[i] = ipiv[i]; }
   __syncthreads();
   if (tid == 0)
     for (int j = 0; j < n; ++j) {
-      const int p = piv[j], a = perm[j], b = perm[p];
+      const int p = piv[j];
+      const unsigned short a = perm[j], b = perm[p];
       perm[j] = b; perm[p] = a;
     }
   __syncthreads();
@@ -578,30 +579,30 @@ __global__ void __launch_bounds__(kNarrowThreads) getrs_narrow_kernel(const Cx<R
     const bool fwd = sweep == 0;                              // L (unit lower), then U (upper)
     auto begin = [&](int b) { return fwd ? b * NB : max(0, n - (b + 1) * NB); };
     auto size = [&](int b) { return fwd ? min(NB, n - b * NB) : (n - b * NB) - begin(b); };
-    auto bring = [&](int b, int buf) {                        // block b's diagonal (its owner)
+    auto bring = [&](int b) {                                 // block b's diagonal (its owner)
       const int i0 = begin(b), ib = size(b);
       for (int e = tid; e < NB * NB; e += nt) {
         const int r = e % NB, t = e / NB;
-        sD[buf][t][r] = (r < ib && t < ib) ? LU[i0 + r + (long long)(i0 + t) * lda] : cxzero<R>();
+        sD[t][r] = (r < ib && t < ib) ? LU[i0 + r + (long long)(i0 + t) * lda] : cxzero<R>();
       }
     };
-    if (rank == 0) bring(0, 0);
+    if (rank == 0) bring(0);
     __syncthreads();
     for (int b = 0; b < nblk; ++b) {
-      const int i0 = begin(b), ib = size(b), buf = b & 1;
+      const int i0 = begin(b), ib = size(b);
       if (rank == (unsigned)(b % (int)ctas) && warp < NC) {
         C_* xc = X + (size_t)warp * n + i0;
         C_ x = lane < ib ? xc[lane] : cxzero<R>();
         if (fwd) {
           for (int t = 0; t < ib; ++t) {
-            const C_ l = sD[buf][t][lane], xt = shf(x, t);
+            const C_ l = sD[t][lane], xt = shf(x, t);
             if (lane > t) x = sub_mul<kUpdate>(x, l, xt);
           }
         } else {
           Divisor<R> dv;
-          dv.set(lane < ib ? sD[buf][lane][lane] : cxone<R>());
+          dv.set(lane < ib ? sD[lane][lane] : cxone<R>());
           for (int t = ib - 1; t >= 0; --t) {
-            const C_ u = sD[buf][t][lane];
+            const C_ u = sD[t][lane];
             if (lane == t) x = dv.of(x);
             __syncwarp();
             const C_ xt = shf(x, t);
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(kNarrowThreads) getrs_narrow_kernel(const Cx<R
       barrier_all(ctas);
       // the block's part of the blocks still to solve (CTA k's: k, k + C, ...)
       const int nb = b + 1;
-      if (nb < nblk && rank == (unsigned)(nb % (int)ctas)) bring(nb, buf ^ 1);
+      if (nb < nblk && rank == (unsigned)(nb % (int)ctas)) bring(nb);
       const int first = nb + (int)((rank + ctas - (unsigned)(nb % (int)ctas)) % ctas);
       const int mine = first < nblk ? (nblk - first + (int)ctas - 1) / (int)ctas : 0;
       for (int q = warp; q < mine * G; q += nw) {
