@@ -723,14 +723,15 @@ __global__ void __launch_bounds__(1024) unghr_kernel(Cx<R>* __restrict__ Aall, i
 }
 
 // ---------------------------------------------------------- 3. Schur form by shifted QR: wb_qr.cuh
-// FP64 matrices of up to kQrSmall, and double-float batches past the GPU, take the sweep element by
+// FP64 matrices of up to kQrSmall, and some double-float ones (qr_small), take the sweep element by
 // element, one CTA a matrix and one barrier a reflector: the windows of wb_qr.cuh are 16 reflectors wide
 // and their two ticks a sweep (a window, and its far updates before the next sweep) cost more there. The
 // FP64 ones are the 32 x 32 group blocks of the mixed form's Newton steps, most of them diagonal.
 constexpr int kQrSmall = 32;
 
-template <class R>
-__global__ void __launch_bounds__(256) hseqr_small_kernel(Cx<R>* __restrict__ Hall, int n, int ldh,
+// MT, its largest CTA, sets the registers: 85 a thread for 768, so that CTAs run side by side; 255 for 256.
+template <class R, int MT>
+__global__ void __launch_bounds__(MT) hseqr_small_kernel(Cx<R>* __restrict__ Hall, int n, int ldh,
                                                             long long h_bs, Cx<R>* __restrict__ Zall, int ldz,
                                                             long long z_bs, Cx<R>* __restrict__ w_all,
                                                             int32_t* __restrict__ status, int st_div, int itmax, const int* __restrict__ live) {
@@ -1106,6 +1107,34 @@ template <class R> static QrShape qr_shape(int batch, int n) {
   return s;
 }
 
+// The element-by-element sweep where it is taken (threads, 0 where not; wide: by the instance with 255 registers): FP64
+// matrices of up to kQrSmall, and of double-float (the same bits either way; modes in ms, so against in windows)
+//   n <= 22: one matrix of 14 / 18 1.5 / 2.4 against 1.8 / 2.8;
+//   more matrices than SMs: 600 of 50 / 126 / 242 24 / 169 / 1080 against 35 / 228 / 1260. 256 threads where a matrix keeps
+//     them busy and three such CTAs an SM hold the batch (400 of 70: 45 against 48 by 128); else 128, four an SM with 255
+//     registers or six with 85, 1.4 times as long: whichever takes its waves in less (600 / 1500 of 66: 47 / 128 and
+//     63 / 123); from n = 126 on the four (200 of 162 / 242: 202 / 526; 205 / 557 with 85; 287 / 679 by 512);
+//   one matrix an SM from n = 144 on, by as many threads as have pairs: 152 of 162 / 242 / 450 173 / 394 / 1714 against
+//     185 / 424 / 2219; where windows still have two CTAs' room they win below n = 400 (100 of 202: 205 against 198;
+//     of 450: 1595 against 1777).
+struct QrSmall { int threads; bool wide; };
+template <class R> static QrSmall qr_small(int batch, int n) {
+  const bool fp64 = std::is_same<R, double>::value;
+  const int sms = sm_count();
+  const bool past = batch > sms, each = n >= 144 && 4LL * batch > (n >= 400 ? 2LL : 3LL) * sms;
+  if (!(fp64 ? n <= kQrSmall : n <= 22 || past || each)) return {0, false};
+  const bool busy = past && n > 64 && n < 126 && batch <= 3 * sms;            // 256 threads
+  const int fours = (batch + 4 * sms - 1) / (4 * sms), sixes = (batch + 6 * sms - 1) / (6 * sms);
+  const bool wide = fp64 || (past && !busy && (n >= 126 || 10 * fours <= 14 * sixes));
+  const int most = wide ? 256 : 768, forced = tuning(kTuneQrThreads);
+  if (forced >= 64 && forced % 32 == 0) return {forced < most ? forced : most, wide};
+  if (n <= 64) return {128, wide};
+  if (past) return {busy ? 256 : 128, wide};
+  int t = most;
+  while (t > 128 && t / 2 >= 2 * n) t /= 2;
+  return {t, wide};
+}
+
 // Threads of one Hessenberg-reduction (and Q-forming) CTA: one warp per trailing column, so as
 // many warps as fit when few matrices share an SM. WB_TUNE_HRD_THREADS overrides the choice.
 int hrd_threads(int batch, int n) {
@@ -1259,12 +1288,14 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
   if (timed) cudaEventRecord(e0, s);
   bool launched = false;
   if constexpr (sizeof(R) > 4) {
-    // the element-by-element sweep: small FP64 matrices, and double-float ones that fill the GPU (the same bits;
-    // modes of 600 matrices of 50 / 126 / 242: 24 / 169 / 1080 ms against 35 / 228 / 1260 in windows)
-    if (std::is_same<R, double>::value ? n <= kQrSmall : batch > sm_count()) {
-      allow_shared(hseqr_small_kernel<R>, kVectorShared / 2);
-      hseqr_small_kernel<R><<<batch, 128, (size_t)n * sizeof(Cx<R>), s>>>(A, n, lda, a_bs, Z, ldz, z_bs, w, status,
-                                                                         st_div < 1 ? 1 : st_div, itmax, live);
+    const QrSmall small = qr_small<R>(batch, n);
+    if (small.threads) {
+      auto kernel = hseqr_small_kernel<R, 256>;
+      if constexpr (!std::is_same<R, double>::value)
+        if (!small.wide) kernel = hseqr_small_kernel<R, 768>;
+      allow_shared(kernel, kVectorShared / 2);
+      kernel<<<batch, small.threads, (size_t)n * sizeof(Cx<R>), s>>>(A, n, lda, a_bs, Z, ldz, z_bs, w, status,
+                                                                    st_div < 1 ? 1 : st_div, itmax, live);
       launched = true;
     }
   }
