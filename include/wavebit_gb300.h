@@ -272,12 +272,14 @@ long long wb_kernel_launches(wb_handle* h);
 
 /* Launch-shape tunables, process-wide: 0 restores the library's own choice. The autotuner
  * (wavebit_gb300/autotune.py) times candidates per (orders, layers, batch) bucket and sets them
- * before each batch. Thread counts never change a result; WB_TUNE_TENSOR_CORES = 1 moves the
+ * before each batch. Thread counts never change a result, but for its last bits: WB_TUNE_HRD_THREADS sets
+ * the order of one sum in the reductions that take it. WB_TUNE_TENSOR_CORES = 1 moves the
  * complex products from the tensor cores (FP32: split TF32; FP64: exact slices) to FP32 and FP64 SIMT,
  * which changes their rounding within FP32 (FP64) accuracy. No counterpart in the reference (its backends leave launch shapes to
  * LAPACK and torch). */
 #define WB_TUNE_QR_THREADS 0     /* threads of a QR-sweep CTA (64..1024, multiple of 32; held to 128..512 in
-                                    FP32 and 128..256 in the other forms) */
+                                    FP32 and 128..256 in the other forms; 64..256 and, in double-float,
+                                    64..768 where it runs element by element) */
 #define WB_TUNE_HRD_THREADS 1    /* threads of a Hessenberg-reduction CTA (64..1024, multiple of 32); FP64 matrices
                                     of 33..512 take 256 */
 #define WB_TUNE_LU_THREADS 2     /* reserved: threads of an LU / triangular-solve CTA */

@@ -9,12 +9,13 @@ the tuner times candidate settings of the launch-shape tunables that ``wb_set_tu
 It searches by coordinate descent from the library's own choice (0), one tunable at a time,
 keeping a candidate only when it is faster by more than ``min_gain``. The choices are persisted
 in a JSON file keyed by bucket, so that a server tunes offline and applies them at run time.
-These tunables change launch shapes only, never a result. ``tune_batch_limit`` picks, among batch
-sizes that fit a worker's memory share, the one with the most solves per second.
+These tunables change launch shapes only, never a result past its last bits (``hrd_threads`` sets the
+order of one sum in the Hessenberg reductions that take it). ``tune_batch_limit`` picks, among
+batch sizes that fit a worker's memory share, the one with the most solves per second.
 
 The tunables are process-wide. A server whose workers run different buckets at once applies each
 bucket's choice before launching it. A concurrent launch may then run with another bucket's
-shape, which costs time but never changes an answer.
+shape, which costs time but never changes an answer past its last bits.
 
     python -m wavebit_gb300.autotune --orders 12 --layers 4 --batch 38 --precision mixed --path tuning.json
 """
@@ -28,6 +29,25 @@ KNOBS = {
     'qr_threads': (0, (0, 256, 384, 512, 768)),
     'hrd_threads': (1, (0, 256, 512, 1024)),
 }
+#: the largest QR-sweep CTA of a form whose larger candidates would all launch that one again
+QR_MOST = {'double': 256, 'fp64': 256, 'mixed': 512}
+
+
+def candidates(name, key):
+    """The values of a tunable that launch differently in bucket ``key``: a form's sweep has a largest CTA, and
+    the FP64 Hessenberg reduction has one shape for matrices of 33 to 512."""
+    values = KNOBS[name][1]
+    try:
+        orders, form = key.split('/')[0], key.split('/')[-1]
+        hu, hv = (int(v) for v in orders.split('x'))
+    except ValueError:
+        return values
+    n = 2 * (2 * hu + 1) * (2 * hv + 1)
+    if name == 'qr_threads' and form in QR_MOST:
+        return tuple(v for v in values if v <= QR_MOST[form])
+    if name == 'hrd_threads' and form in ('double', 'fp64') and 33 <= n <= 512:
+        return (0,)
+    return values
 
 
 def bucket_key(orders, layers, batch, precision):
@@ -109,7 +129,7 @@ class Autotuner:
         t_best = self._time(run)
         trials = [{'settings': dict(best), 'seconds': t_best}]
         for name in names:
-            for v in KNOBS[name][1]:
+            for v in candidates(name, key):
                 if v == best[name]:
                     continue
                 cand = dict(best, **{name: v})
