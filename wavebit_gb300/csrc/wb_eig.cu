@@ -277,10 +277,10 @@ __device__ __forceinline__ Cx<float> row_times(const Cx<float>* ar, int lda, con
   return acc + cxmk<float>(__shfl_xor_sync(0xffffffffu, acc.x, 1), __shfl_xor_sync(0xffffffffu, acc.y, 1));
 }
 
-template <class R>
-__global__ void __launch_bounds__(1024) gehrd_panel_kernel(Cx<R>* __restrict__ Aall, int n, int lda, long long a_bs,
-                                                           Cx<R>* __restrict__ tau_all, int k, int bb,
-                                                           Cx<R>* __restrict__ Wsall, long long ws_bs) {
+__global__ void __launch_bounds__(1024) gehrd_panel_kernel(Cx<float>* __restrict__ Aall, int n, int lda, long long a_bs,
+                                                           Cx<float>* __restrict__ tau_all, int k, int bb,
+                                                           Cx<float>* __restrict__ Wsall, long long ws_bs) {
+  using R = float;
   using C_ = Cx<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   C_* sb = reinterpret_cast<C_*>(smraw);          // (n) the column being reduced
@@ -387,38 +387,18 @@ __global__ void __launch_bounds__(1024) gehrd_panel_kernel(Cx<R>* __restrict__ A
     }
     if (tid == 0) T[j][j] = tj;
     __syncthreads();
-    // Y[:, j] = tau (A[:, c+1:] v[c+1:] - Y_j w2): four threads a row in FP32 (eight loads in flight each: a
-    // thread a row and four loads ran on their latency), one row per thread in the other forms
+    // Y[:, j] = tau (A[:, c+1:] v[c+1:] - Y_j w2): four threads a row, eight loads in flight each (a
+    // thread a row and four loads ran on their latency)
     const int m = n - c - 1;
-    if constexpr (sizeof(R) == 4) {
-      for (int i0 = 0; i0 < n; i0 += nt / 4) {
-        const int r = i0 + (tid >> 2);
-        const bool in = r < n;
-        C_ y = row_times<8>(A + (in ? r : 0) + (long long)(c + 1) * lda, lda, sv + c + 1, m);
-        if (in && (tid & 3) == 0) {
+    for (int i0 = 0; i0 < n; i0 += nt / 4) {
+      const int r = i0 + (tid >> 2);
+      const bool in = r < n;
+      C_ y = row_times<8>(A + (in ? r : 0) + (long long)(c + 1) * lda, lda, sv + c + 1, m);
+      if (in && (tid & 3) == 0) {
 #pragma unroll 8
-          for (int l = 0; l < j; ++l) y = y - Y[r + (long long)l * n] * s_w[l];
-          Y[r + (long long)j * n] = ident ? cxzero<R>() : tj * y;
-        }
+        for (int l = 0; l < j; ++l) y = y - Y[r + (long long)l * n] * s_w[l];
+        Y[r + (long long)j * n] = ident ? cxzero<R>() : tj * y;
       }
-    } else
-    for (int r = tid; r < n; r += nt) {
-      const C_* ar = A + r + (long long)(c + 1) * lda;
-      const C_* vv = sv + c + 1;
-      C_ acc0 = cxzero<R>(), acc1 = cxzero<R>(), acc2 = cxzero<R>(), acc3 = cxzero<R>();
-      int q = 0;
-      for (; q + 3 < m; q += 4) {
-        const C_ a0 = ar[(long long)q * lda], a1 = ar[(long long)(q + 1) * lda];
-        const C_ a2 = ar[(long long)(q + 2) * lda], a3 = ar[(long long)(q + 3) * lda];
-        acc0 = cxfma(a0, vv[q], acc0);
-        acc1 = cxfma(a1, vv[q + 1], acc1);
-        acc2 = cxfma(a2, vv[q + 2], acc2);
-        acc3 = cxfma(a3, vv[q + 3], acc3);
-      }
-      for (; q < m; ++q) acc0 = cxfma(ar[(long long)q * lda], vv[q], acc0);
-      C_ y = (acc0 + acc2) + (acc1 + acc3);
-      for (int l = 0; l < j; ++l) y = y - Y[r + (long long)l * n] * s_w[l];
-      Y[r + (long long)j * n] = ident ? cxzero<R>() : tj * y;
     }
     __syncthreads();
   }
@@ -609,10 +589,10 @@ __global__ void __launch_bounds__(kHrdClusterThreads) gehrd_panel_cluster_kernel
 // forward: T[:j, j] = -tau_j T_j V_j^H v_j, T[j, j] = tau_j), and Z's trailing block gets
 // Z <- Z - V (T (V^H Z)) as batched products. This kernel writes the panel's V, conj(V) (n x
 // kHrdPanel) and T (column-major kHrdPanel x kHrdPanel) into the scratch.
-template <class R>
-__global__ void __launch_bounds__(1024) unghr_panel_kernel(const Cx<R>* __restrict__ Aall, int n, int lda,
-                                                           long long a_bs, const Cx<R>* __restrict__ tau_all, int k0,
-                                                           int bb, Cx<R>* __restrict__ Wsall, long long ws_bs) {
+__global__ void __launch_bounds__(1024) unghr_panel_kernel(const Cx<float>* __restrict__ Aall, int n, int lda,
+                                                           long long a_bs, const Cx<float>* __restrict__ tau_all, int k0,
+                                                           int bb, Cx<float>* __restrict__ Wsall, long long ws_bs) {
+  using R = float;
   using C_ = Cx<R>;
   __shared__ C_ T[kHrdPanel][kHrdPanel + 1];
   __shared__ C_ s_w[kHrdPanel];
@@ -1191,6 +1171,60 @@ static bool reduce64(cudaStream_t s, int batch, int n, Cx<double>* A, int lda, l
   return true;
 }
 
+// FP32: H in panels (ws: the panels' scratch), Q in panels
+static void reduce_panels(cudaStream_t s, int batch, int n, Cx<float>* A, int lda, long long a_bs, Cx<float>* ws,
+                          long long ws_bs, Cx<float>* tau, int th) {
+  using C_ = Cx<float>;
+  constexpr int BB = kHrdPanel, most = 200 * 1024;
+  allow_shared(gehrd_panel_kernel, kVectorShared / 2);
+  const long long nB = (long long)n * BB;
+  C_ *V = ws, *Vc = ws + nB, *Y = ws + 2 * nB, *Wm = ws + 3 * nB, *Xm = ws + 4 * nB, *TH = ws + 5 * nB;
+  const double2 one = make_double2(1.0, 0.0), mone = make_double2(-1.0, 0.0), zero = make_double2(0.0, 0.0);
+  int ctas = 1;
+  while (2 * ctas <= 8 && 2LL * ctas * batch <= sm_count()) ctas *= 2;
+  const size_t spread = hrd_panel_shared(n, ctas), sm = 2 * (size_t)n * sizeof(C_);
+  for (int k = 0; k + 2 < n; k += BB) {
+    const int bb = min(BB, n - 2 - k);
+    if (ctas > 1 && spread <= most) {
+      launch_cluster(s, gehrd_panel_cluster_kernel, most, ctas, batch, kHrdClusterThreads, spread, A, n, lda, a_bs, tau, k, bb,
+                     ws, ws_bs, th);
+    } else {
+      gehrd_panel_kernel<<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, k, bb, ws, ws_bs); note_launch();
+    }
+    const int c0 = k + bb, m = n - c0, rows = n - k - 1;
+    if (m <= 0) continue;
+    C_* Ac = A + (long long)c0 * lda;
+    // A[:, c0:] -= Y conj(V[c0:, :])^T
+    gemm<float>(s, batch, n, m, bb, mone, Y, 1, n, ws_bs, Vc + c0, n, 1, ws_bs, one, Ac, 1, lda, a_bs);
+    // W = V[k+1:, :]^H A[k+1:, c0:];  X = T^H W;  A[k+1:, c0:] -= V[k+1:, :] X
+    gemm<float>(s, batch, bb, m, rows, one, Vc + (k + 1), n, 1, ws_bs, Ac + (k + 1), 1, lda, a_bs, zero, Wm, 1, BB, ws_bs);
+    gemm<float>(s, batch, bb, m, bb, one, TH, 1, BB, ws_bs, Wm, 1, BB, ws_bs, zero, Xm, 1, BB, ws_bs);
+    gemm<float>(s, batch, rows, m, bb, mone, V + (k + 1), 1, n, ws_bs, Xm, 1, BB, ws_bs, one, Ac + (k + 1), 1, lda, a_bs);
+  }
+}
+
+static void form_panels(cudaStream_t s, int batch, int n, Cx<float>* A, int lda, long long a_bs, Cx<float>* Z, int ldz,
+                        long long z_bs, const Cx<float>* tau, Cx<float>* ws, long long ws_bs, int th) {
+  using C_ = Cx<float>;
+  constexpr int BB = kHrdPanel;
+  const long long nB = (long long)n * BB;
+  C_ *V = ws, *Vc = ws + nB, *Wm = ws + 2 * nB, *Xm = ws + 3 * nB, *Tm = ws + 4 * nB;
+  const double2 one = make_double2(1.0, 0.0), mone = make_double2(-1.0, 0.0), zero = make_double2(0.0, 0.0);
+  set_identity<float>(s, batch, n, Z, ldz, z_bs);
+  const int nk = n - 2;                                    // reflectors 0 .. n - 3
+  for (int k0 = ((nk - 1) / BB) * BB; k0 >= 0; k0 -= BB) {
+    const int bb = min(BB, nk - k0), rows = n - k0 - 1;
+    unghr_panel_kernel<<<batch, th, 0, s>>>(A, n, lda, a_bs, tau, k0, bb, ws, ws_bs); note_launch();
+    C_* Zb = Z + (k0 + 1) + (long long)(k0 + 1) * ldz;
+    // W = V[k0+1:, :]^H Z_blk;  X = T W;  Z_blk -= V[k0+1:, :] X
+    gemm<float>(s, batch, bb, rows, rows, one, Vc + (k0 + 1), n, 1, ws_bs, Zb, 1, ldz, z_bs, zero, Wm, 1, BB, ws_bs);
+    gemm<float>(s, batch, bb, rows, bb, one, Tm, 1, BB, ws_bs, Wm, 1, BB, ws_bs, zero, Xm, 1, BB, ws_bs);
+    gemm<float>(s, batch, rows, rows, bb, mone, V + (k0 + 1), 1, n, ws_bs, Xm, 1, BB, ws_bs, one, Zb, 1, ldz, z_bs);
+  }
+  const unsigned gx = (unsigned)min((long long)sm_count(), ((long long)n * n + 255) / 256);
+  clear_below_subdiag_kernel<float><<<dim3(gx, batch), 256, 0, s>>>(A, n, lda, a_bs); note_launch();
+}
+
 template <class R>
 void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a_bs, Cx<R>* Z, int ldz,
                 long long z_bs, Cx<R>* w, Cx<R>* tau, int32_t* status, int st_div, Cx<R>* ws, long long ws_bs,
@@ -1200,80 +1234,23 @@ void geev_schur(cudaStream_t s, int batch, int n, Cx<R>* A, int lda, long long a
   allow_shared(gehrd_kernel<R>, kVectorShared);
   allow_shared(unghr_kernel<R>, kVectorShared);
   const int th = hrd_threads(batch, n);
+  bool hessenberg = false, formed = false;                 // H, Q
+  if constexpr (std::is_same<R, double>::value)
+    if (n > kQrSmall) hessenberg = formed = reduce64(s, batch, n, A, lda, a_bs, Z, ldz, z_bs, tau);
   // the FP32 form at n >= 192 reduces in panels (Z, not yet formed, holds the panels' scratch:
   // 5 n kHrdPanel + kHrdPanel^2 elements, within n * ldz from n = 161 on)
-  const bool blocked = sizeof(R) == 4 && n >= 192 && ldz >= n && tuning(kTuneHrdBlocked) != 1;
-  bool reduced = false;
-  if constexpr (std::is_same<R, double>::value) {
-    if (n > kQrSmall) reduced = reduce64(s, batch, n, A, lda, a_bs, Z, ldz, z_bs, tau);
-  }
-  if (reduced) {
-  } else if (blocked) {
-    allow_shared(gehrd_panel_kernel<R>, kVectorShared / 2);
-    const int BB = kHrdPanel;
-    const long long nB = (long long)n * BB;
-    Cx<R>* V = Z;
-    Cx<R>* Vc = Z + nB;
-    Cx<R>* Y = Z + 2 * nB;
-    Cx<R>* Wm = Z + 3 * nB;
-    Cx<R>* Xm = Z + 4 * nB;
-    Cx<R>* TH = Z + 5 * nB;
-    const double2 one = make_double2(1.0, 0.0), mone = make_double2(-1.0, 0.0), zero = make_double2(0.0, 0.0);
-    for (int k = 0; k + 2 < n; k += BB) {
-      const int bb = min(BB, n - 2 - k);
-      bool spread = false;
-      if constexpr (sizeof(R) == 4) {
-        int c = 1;
-        while (2 * c <= 8 && 2LL * c * batch <= sm_count()) c *= 2;
-        const size_t smc = hrd_panel_shared(n, c);
-        constexpr int most = 200 * 1024;
-        if (c > 1 && smc <= most) {
-          launch_cluster(s, gehrd_panel_cluster_kernel, most, c, batch, kHrdClusterThreads, smc, A, n, lda, a_bs, tau, k, bb,
-                         Z, z_bs, th);
-          spread = true;
-        }
+  if constexpr (std::is_same<R, float>::value)
+    if (n >= 192 && ldz >= n && tuning(kTuneHrdBlocked) != 1) {
+      reduce_panels(s, batch, n, A, lda, a_bs, Z, z_bs, tau, th);
+      hessenberg = true;
+      // Q in panels when the caller lends scratch (5 n kHrdPanel + kHrdPanel^2 elements a matrix)
+      if (ws && ws_bs >= 5LL * n * kHrdPanel + kHrdPanel * kHrdPanel) {
+        form_panels(s, batch, n, A, lda, a_bs, Z, ldz, z_bs, tau, ws, ws_bs, th);
+        formed = true;
       }
-      if (!spread) { gehrd_panel_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, k, bb, Z, z_bs); note_launch(); }
-      const int c0 = k + bb, m = n - c0, rows = n - k - 1;
-      if (m <= 0) continue;
-      Cx<R>* Ac = A + (long long)c0 * lda;
-      // A[:, c0:] -= Y conj(V[c0:, :])^T
-      gemm<R>(s, batch, n, m, bb, mone, Y, 1, n, z_bs, Vc + c0, n, 1, z_bs, one, Ac, 1, lda, a_bs);
-      // W = V[k+1:, :]^H A[k+1:, c0:];  X = T^H W;  A[k+1:, c0:] -= V[k+1:, :] X
-      gemm<R>(s, batch, bb, m, rows, one, Vc + (k + 1), n, 1, z_bs, Ac + (k + 1), 1, lda, a_bs, zero, Wm, 1, BB, z_bs);
-      gemm<R>(s, batch, bb, m, bb, one, TH, 1, BB, z_bs, Wm, 1, BB, z_bs, zero, Xm, 1, BB, z_bs);
-      gemm<R>(s, batch, rows, m, bb, mone, V + (k + 1), 1, n, z_bs, Xm, 1, BB, z_bs, one, Ac + (k + 1), 1, lda, a_bs);
     }
-  } else {
-    gehrd_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, live); note_launch();
-  }
-  // Q in panels when the caller lends scratch (5 n kHrdPanel + kHrdPanel^2 elements a matrix)
-  if (reduced) {
-  } else if (blocked && ws && ws_bs >= 5LL * n * kHrdPanel + kHrdPanel * kHrdPanel) {
-    const int BB = kHrdPanel;
-    const long long nB = (long long)n * BB;
-    Cx<R>* V = ws;
-    Cx<R>* Vc = ws + nB;
-    Cx<R>* Wm = ws + 2 * nB;
-    Cx<R>* Xm = ws + 3 * nB;
-    Cx<R>* Tm = ws + 4 * nB;
-    const double2 one = make_double2(1.0, 0.0), mone = make_double2(-1.0, 0.0), zero = make_double2(0.0, 0.0);
-    set_identity<R>(s, batch, n, Z, ldz, z_bs);
-    const int nk = n - 2;                                  // reflectors 0 .. n - 3
-    for (int k0 = ((nk - 1) / BB) * BB; k0 >= 0; k0 -= BB) {
-      const int bb = min(BB, nk - k0), rows = n - k0 - 1;
-      unghr_panel_kernel<R><<<batch, th, 0, s>>>(A, n, lda, a_bs, tau, k0, bb, ws, ws_bs); note_launch();
-      Cx<R>* Zb = Z + (k0 + 1) + (long long)(k0 + 1) * ldz;
-      // W = V[k0+1:, :]^H Z_blk;  X = T W;  Z_blk -= V[k0+1:, :] X
-      gemm<R>(s, batch, bb, rows, rows, one, Vc + (k0 + 1), n, 1, ws_bs, Zb, 1, ldz, z_bs, zero, Wm, 1, BB, ws_bs);
-      gemm<R>(s, batch, bb, rows, bb, one, Tm, 1, BB, ws_bs, Wm, 1, BB, ws_bs, zero, Xm, 1, BB, ws_bs);
-      gemm<R>(s, batch, rows, rows, bb, mone, V + (k0 + 1), 1, n, ws_bs, Xm, 1, BB, ws_bs, one, Zb, 1, ldz, z_bs);
-    }
-    const unsigned gx = (unsigned)min((long long)sm_count(), ((long long)n * n + 255) / 256);
-    clear_below_subdiag_kernel<R><<<dim3(gx, batch), 256, 0, s>>>(A, n, lda, a_bs); note_launch();
-  } else {
-    unghr_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, Z, ldz, z_bs, live); note_launch();
-  }
+  if (!hessenberg) { gehrd_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, live); note_launch(); }
+  if (!formed) { unghr_kernel<R><<<batch, th, sm, s>>>(A, n, lda, a_bs, tau, Z, ldz, z_bs, live); note_launch(); }
   int itmax = 30 * (n > 10 ? n : 10);
   const QrShape shape = qr_shape<R>(batch, n);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
