@@ -35,8 +35,8 @@
 //
 // What bounds it: a tile's own latencies. One CTA an SM (192 KB, all of tensor memory) takes about 17 us a
 // tile of K = 64: the scales' pass, the splitting and the 288 MMAs (5 us alone), the eight accumulators'
-// assembly, and C read and written; FP64 FMAs take 270 us. 450 x 450 x 64, 8 matrices, C read and written: 128 us
-// (6.5 TFLOP/s), 121 without the k's scales; x 450 769 us (7.6), 713 without; K = 31 the same with and without.
+// assembly, and C read and written; FP64 FMAs take 270 us. 450 x 450 x 64, 8 matrices, C read and written: 126 us
+// (6.6 TFLOP/s), 121 without the k's scales; x 450 5% longer with them too; K = 31 the same with and without.
 // Holding C's entries during the MMAs spills at 168 registers and was 10% slower.
 // Every mbarrier wait is bounded, as in wb_tc.cuh.
 #pragma once
@@ -73,9 +73,9 @@ constexpr int kOff = 4096, kBad = 1 << 20;
 // the shift of a k that contributes nothing (its column of A or row of B is zero)
 constexpr int kDropped = -30000;
 
-// The exponent of a complex entry's larger component, biased, + kSub so that subnormals' (by their leading bit,
-// down to -51) stay positive; 0 for zero.
-constexpr int kSub = 64;
+// The exponent of a complex entry's larger component, biased (subnormals' by their leading bit, down to -51),
+// + kSub; 0 for zero, which stays below kSome under any shift, as no other entry does but a dropped one.
+constexpr int kSub = 8192 + 64, kSome = 6144;
 __device__ __forceinline__ int entry_exponent(double2 v) {
   const int hx = __double2hiint(v.x) & 0x7fffffff, hy = __double2hiint(v.y) & 0x7fffffff;
   const int e = max(hx, hy) >> 20;
@@ -248,15 +248,13 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
     if (!issuer) {
       // the largest of the warp's 32 lines for each of its k, 16 at a time: pairs of 16 bits, halved from lane to
       // lane until a lane holds one pair
-      const uint32_t base = (uint32_t)(kOff - s_top[side + line]);
+      const int own = s_top[side + line];
+      const uint32_t base = own ? (uint32_t)(kSub + kOff - own) * 0x10001u : 0u;
 #pragma unroll 1
       for (int t0 = 0; t0 < tk; t0 += 16) {
         uint32_t w[8];
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          const uint32_t e = ex[kWorkers * (t0 / 2 + t)];
-          w[t] = ((e & 0xffffu) ? (e & 0xffffu) + base : 0u) | ((e >> 16) ? ((e >> 16) + base) << 16 : 0u);
-        }
+        for (int t = 0; t < 8; ++t) w[t] = ex[kWorkers * (t0 / 2 + t)] + base;
 #pragma unroll
         for (int h = 4, bit = 1; h >= 1; h >>= 1, bit <<= 1)
 #pragma unroll
@@ -269,7 +267,7 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
         w[0] = __vmaxu2(w[0], __shfl_xor_sync(0xffffffffu, w[0], 16));
         const int t = t0 + (((lane & 1) << 3) | ((lane & 2) << 1) | ((lane & 4) >> 1) | (lane >> 4));
         const int m = (int)(lane >> 4 ? w[0] >> 16 : w[0] & 0xffffu);
-        if (m && !(lane & 8)) atomicMax(&s_k[side + part + 2 * t], m);
+        if (m >= kSub && !(lane & 8)) atomicMax(&s_k[side + part + 2 * t], m);
       }
     }
     __syncthreads();
@@ -281,18 +279,16 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
     }
     __syncthreads();
     if (!issuer) {
-      int mx = kDropped;
+      uint32_t most = (uint32_t)(kDropped & 0xffff) * 0x10001u;
 #pragma unroll 1
       for (int t = 0; t < tk; t += 8) {
         const uint4 sv = *reinterpret_cast<const uint4*>(s_half + side + part * 32 + t);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const uint32_t e = ex[kWorkers * (t / 2 + u)], h = u == 0 ? sv.x : u == 1 ? sv.y : u == 2 ? sv.z : sv.w;
-          if (e & 0xffffu) mx = max(mx, (int)(e & 0xffffu) + (short)h);
-          if (e >> 16) mx = max(mx, (int)(e >> 16) + ((int)h >> 16));
-        }
+        for (int u = 0; u < 4; ++u)
+          most = __viaddmax_s16x2(ex[kWorkers * (t / 2 + u)], u == 0 ? sv.x : u == 1 ? sv.y : u == 2 ? sv.z : sv.w, most);
       }
-      mx += kOff - kSub;
+      int mx = max((int)(short)most, (int)most >> 16);
+      mx = mx >= kSome ? mx - kSub + kOff : 0;
       if (bad) mx = kBad;
       if (mx > 0) atomicMax(&s_line[side + line], mx);
     }
