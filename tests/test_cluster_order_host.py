@@ -120,3 +120,14 @@ def test_narrow_solve_has_one_answer_whatever_cta_runs_first(n, ctas):
     # without the meeting the model finds the conflict
     if ctas > 1:
         assert any(_run(LU, b, ctas, 4, order, False)[1] for order in itertools.permutations(range(ctas)))
+
+
+def test_the_sliced_product_leaves_at_one_barrier():
+    """A flag that thread 0 sets when a wait runs out is read by every thread after the next barrier, and not set again
+    before a barrier after that: set by the next chunk's wait, a late warp could read it for this chunk's and leave
+    where the others stay. So two chunks in a row, and a panel's end, have flags of their own."""
+    body = _body(open(os.path.join(CSRC, 'wb_oz.cuh')).read(), 'zgemm_kernel')
+    reads = re.findall(r'if \(s_fail\[(\w+)\]\) \{ ok = false; break; \}', body)
+    sets = re.findall(r's_fail\[(\w+)\] = 1;', body)
+    assert reads == ['buf', '2'] and sorted(sets) == ['2', 'buf'] and 'const int buf = uses & 1' in body
+    assert not re.search(r's_fail\b(?!\[)', body)

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t bars[2];
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_fail;
+  __shared__ int s_fail[3];                                    // thread 0's wait ran out: by a chunk's buffer, a panel's end
   __shared__ int s_top[2 * kT], s_line[2 * kT];                // the lines' exponents before and after the k's shifts
   __shared__ int s_k[2 * kT];                                  // a k's largest entry, against its line's largest
   __shared__ __align__(16) short s_shift[2 * kT];              // its shift
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
     tc::mbar_init(&bars[0]);
     tc::mbar_init(&bars[1]);
     asm volatile("fence.mbarrier_init.release.cluster;");
-    s_fail = 0;
+    s_fail[0] = s_fail[1] = s_fail[2] = 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
       const int buf = uses & 1;
       unsigned char* st = smem + buf * kStage;
       if (!issuer) {
-        if (uses >= 2 && tid == 0 && !tc::mbar_wait(&bars[buf], ((uses >> 1) - 1) & 1)) s_fail = 1;
+        if (uses >= 2 && tid == 0 && !tc::mbar_wait(&bars[buf], ((uses >> 1) - 1) & 1)) s_fail[buf] = 1;
         // split: words of 4 digit bytes, high (digits 0..3) and low (4..7), of the 8 real and 8 imaginary parts
         uint32_t rh[8], rl[8], ih[8], il[8];
 #pragma unroll
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
       __syncthreads();
-      if (s_fail) { ok = false; break; }
+      if (s_fail[buf]) { ok = false; break; }                  // (the next chunk's wait sets the other flag)
       if (issuer && lane == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;");
         // descriptors differ by their start address alone (bits 0..13, in 16-byte units)
@@ -368,11 +368,11 @@ __global__ void __launch_bounds__(kThreads) zgemm_kernel(const Args g) {
     if (tid == 0) {
       for (int b = 0; b < 2; ++b) {
         const uint32_t last = uses - 1 - ((uses - 1 - b) & 1);  // the latest chunk in buffer b
-        if (uses > (uint32_t)b && !tc::mbar_wait(&bars[b], (last >> 1) & 1)) s_fail = 1;
+        if (uses > (uint32_t)b && !tc::mbar_wait(&bars[b], (last >> 1) & 1)) s_fail[2] = 1;
       }
     }
     __syncthreads();
-    if (s_fail) { ok = false; break; }
+    if (s_fail[2]) { ok = false; break; }
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (!issuer) {
       const int ea = s_line[arow & 63];
