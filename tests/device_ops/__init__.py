@@ -28,4 +28,5 @@ def load():
         _ops.ops_getrs.argtypes = [i, i, i, p, ll, p, p, i, i]
         _ops.ops_zgemm.argtypes = [i, i, i, i, d, d, p, p, p, i, p, p, i, d, d, p, p]
         _ops.ops_schur.argtypes = [i, i, p, p, p, p, p]
+        _ops.ops_rsqrt.argtypes = [i, p, p, p, p]
     return _ops

@@ -4,7 +4,22 @@
 
 using namespace wb;
 
+namespace {
+__global__ void rsqrt_kernel(int n, const double* v, double* start, double* full, double* cuda) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  start[i] = rsqrt_start(v[i]);
+  full[i] = rsqrt64(v[i]);
+  cuda[i] = rsqrt(v[i]);
+}
+}  // namespace
+
 extern "C" {
+
+int ops_rsqrt(int n, const double* v, double* start, double* full, double* cuda) {
+  rsqrt_kernel<<<(n + 255) / 256, 256>>>(n, v, start, full, cuda);
+  return (int)cudaGetLastError();
+}
 
 int ops_getrf(int is_double, int batch, int n, void* A, long long a_bs, int* piv, int* status) {
   if (is_double) getrf<double>(0, batch, n, (Cx<double>*)A, n, a_bs, piv, n, status, 1);

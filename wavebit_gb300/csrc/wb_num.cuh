@@ -194,7 +194,7 @@ template <class R> WB_ND bool cxfinite(Cx<R> a) { return rfinite(a.x) && rfinite
 template <class R> WB_ND Cx<R> cxfrom(double2 d) { return cxmk<R>(R(d.x), R(d.y)); }
 template <class R> WB_ND double2 cxto(Cx<R> c) { double2 d; d.x = rto(c.x); d.y = rto(c.y); return d; }
 
-// 1 / sqrt(v) to 22 bits for normal v > 0, from the FP32 unit; the exponents by integer operations
+// 1 / sqrt(v) to 2^-21 for normal v > 0, from the FP32 unit (v truncated to FP32); the exponents by integer operations
 // (a conversion costs as much as an FP64 operation, 64 cycles of a scheduler on GB300).
 __device__ __forceinline__ double rsqrt_start(double v) {
   int hi = __double2hiint(v);
@@ -206,7 +206,9 @@ __device__ __forceinline__ double rsqrt_start(double v) {
   return __hiloint2double((int)(b >> 3) + (896 - (k >> 1)) * (1 << 20), (int)(b << 29));
 }
 
-// 1 / sqrt(v): one third-order step from there (the error's cube times 5/16 is below 2^-64)
+// 1 / sqrt(v) = y (1 - d)^(-1/2), d = 1 - v y^2, by the first three terms of the binomial series, 1 + d/2 + 3 d^2/8: with
+// |d| < 2^-20 the next, 5 d^3/16, is below 2^-61. Off by 2 units of 2^-53 at the most: half a unit from the rounding
+// of v y, one from the last addition, the rest from d's terms.
 __device__ __forceinline__ double rsqrt64(double v) {
   const double y = rsqrt_start(v), d = fma(-(v * y), y, 1.0);
   return fma(y, d * fma(d, 0.375, 0.5), y);
