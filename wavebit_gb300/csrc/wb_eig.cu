@@ -1088,31 +1088,36 @@ template <class R> static QrShape qr_shape(int batch, int n) {
 }
 
 // The element-by-element sweep where it is taken (threads, 0 where not; wide: by the instance with 255 registers): FP64
-// matrices of up to kQrSmall, and of double-float (the same bits either way; modes in ms, so against in windows)
-//   n <= 22: one matrix of 14 / 18 1.5 / 2.4 against 1.8 / 2.8;
-//   more matrices than SMs: 600 of 50 / 126 / 242 24 / 169 / 1080 against 35 / 228 / 1260. 256 threads where a matrix keeps
-//     them busy and three such CTAs an SM hold the batch (400 of 70: 45 against 48 by 128); else 128, four an SM with 255
-//     registers or six with 85, 1.4 times as long: whichever takes its waves in less (600 / 1500 of 66: 47 / 128 and
-//     63 / 123); from n = 126 on the four (200 of 162 / 242: 202 / 526; 205 / 557 with 85; 287 / 679 by 512);
-//   one matrix an SM from n = 144 on, by as many threads as have pairs: 152 of 162 / 242 / 450 173 / 394 / 1714 against
-//     185 / 424 / 2219; where windows still have two CTAs' room they win below n = 400 (100 of 202: 205 against 198;
-//     of 450: 1595 against 1777).
+// matrices of up to kQrSmall, and of double-float (the same bits either way; modes in ms)
+//   n <= 22: one matrix of 14 / 18 1.5 / 2.4, in windows 1.8 / 2.8;
+//   one matrix an SM from n = 144 on, by as many threads as have pairs: 152 of 162 / 242 / 450 173 / 394 / 1714, in windows
+//     185 / 424 / 2219; where windows still have two CTAs' room they win below n = 400 (100 of 202: 205, 198 in windows;
+//     of 450: 1595, 1777);
+//   k > 1 matrices an SM (600 of 50 / 126 / 242: 24 / 169 / 1080, in windows 35 / 228 / 1260), by threads and registers that
+//     fill whole waves: 255 registers let two CTAs of 256 threads or four of 128 run side by side, 85 three of 256
+//     or six of 128, each at less.
+//     n >= 126: two wide of 256 for k = 2 (200 of 242: 463; 478 narrow, 536 by 128), four wide of 128 for k = 4 (600 of
+//     450: 5584; 5778 narrow of 256), else three narrow of 256 (450 of 338: 1904; 2111 and 2374 wide; 760 of 242: 1264; 1681, 1443).
+//     n = 65..125: three narrow of 256 for k <= 3 (400 of 70: 45; 48 wide of 128), else four wide or six narrow of 128, 1.4 times
+//     as long, whichever takes its waves in less (600 / 1500 of 66: 47 / 128 and 63 / 123).
 struct QrSmall { int threads; bool wide; };
 template <class R> static QrSmall qr_small(int batch, int n) {
   const bool fp64 = std::is_same<R, double>::value;
-  const int sms = sm_count();
-  const bool past = batch > sms, each = n >= 144 && 4LL * batch > (n >= 400 ? 2LL : 3LL) * sms;
-  if (!(fp64 ? n <= kQrSmall : n <= 22 || past || each)) return {0, false};
-  const bool busy = past && n > 64 && n < 126 && batch <= 3 * sms;            // 256 threads
-  const int fours = (batch + 4 * sms - 1) / (4 * sms), sixes = (batch + 6 * sms - 1) / (6 * sms);
-  const bool wide = fp64 || (past && !busy && (n >= 126 || 10 * fours <= 14 * sixes));
-  const int most = wide ? 256 : 768, forced = tuning(kTuneQrThreads);
-  if (forced >= 64 && forced % 32 == 0) return {forced < most ? forced : most, wide};
-  if (n <= 64) return {128, wide};
-  if (past) return {busy ? 256 : 128, wide};
-  int t = most;
-  while (t > 128 && t / 2 >= 2 * n) t /= 2;
-  return {t, wide};
+  const int sms = sm_count(), k = (batch + sms - 1) / sms;
+  const bool each = n >= 144 && 4LL * batch > (n >= 400 ? 2LL : 3LL) * sms;
+  if (!(fp64 ? n <= kQrSmall : n <= 22 || k > 1 || each)) return {0, false};
+  QrSmall q = {128, fp64};
+  if (!fp64 && k > 1) {
+    if (n >= 126) q = {k == 4 ? 128 : 256, k == 2 || k == 4};
+    else if (n > 64 && k <= 3) q = {256, false};
+    else q = {128, 10 * ((k + 3) / 4) <= 14 * ((k + 5) / 6)};
+  } else if (n > 64) {
+    q = {768, false};
+    while (q.threads > 128 && q.threads / 2 >= 2 * n) q.threads /= 2;
+  }
+  const int most = q.wide ? 256 : 768, forced = tuning(kTuneQrThreads);
+  if (forced >= 64 && forced % 32 == 0) q.threads = forced < most ? forced : most;
+  return q;
 }
 
 // Threads of one Hessenberg-reduction (and Q-forming) CTA: one warp per trailing column, so as
