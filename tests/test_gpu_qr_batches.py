@@ -26,7 +26,7 @@ def test_bits_over_batches_and_shapes(orders, form):
     n = 2 * len(u) * len(v)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     ref = None
-    batches = (1, sms // 2 + 4, sms, sms + 8, 4 * sms + 2) if n <= 70 else (1, sms // 2 + 4, sms, sms + 8)
+    batches = (1, sms // 2 + 4, sms, sms + 8) + ((4 * sms + 2,) if n <= 70 else (2 * sms + 8,) if n < 200 else ())
     for P in batches:
         kx = torch.as_tensor(np.tile(u + 0.13, 2 * hv + 1), device='cuda').expand(P, n // 2).contiguous()
         ky = torch.as_tensor(np.repeat(v + 0.21, 2 * hu + 1), device='cuda').expand(P, n // 2).contiguous()

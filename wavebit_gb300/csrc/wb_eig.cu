@@ -1071,9 +1071,10 @@ template <class R> static QrShape qr_shape(int batch, int n) {
   // More matrices than SMs: small CTAs side by side, as many as the registers take (modes of 600 matrices of
   // 242, FP32: 4 warps 231 ms, 6 206, 8 221; FP64: 4 warps 1.23 s, 5 1.59, 8 1.33), until a tick's far updates
   // outlast its chase and the largest CTA wins (sweep of 512 of 450, FP32: 4 warps 784 ms, 8 656, 16 451;
-  // FP64: 4 warps 5.0 s, 5 8.1, 8 4.2).
+  // FP64: 4 warps 5.0 s, 5 8.1, 8 4.2). In FP64 two of 4 warps fit an SM, so three matrices an SM take one of 8 at a
+  // time (modes of 450 of 162 / 242: 4 warps 417 / 1133 ms, 8 389 / 1027).
   const int cap = sizeof(R) == 4 ? (per_sm <= 1 || n >= 256 ? 16 : per_sm <= 2 ? 7 : 6)
-                                 : (per_sm <= 1 || n >= 320 ? 8 : 4);
+                                 : (per_sm <= 1 || n >= 320 || (per_sm == 3 && n >= 160) ? 8 : 4);
   int warps = (tasks + c - 1) / c + 1;
   warps = warps > cap ? cap : warps < 4 ? 4 : warps;
   QrShape s;
