@@ -542,10 +542,10 @@ __device__ __noinline__ bool near_columns(Cx<R>* H, int ldh, Cx<R>* tile, const 
 //
 // FP32: every lane carries the core (rows and columns k, k + 1) and computes the reflector, lane j
 // the window's column k0 + 2 + j as well; no hand-over is on the chain, which is the core's update
-// and the reflector, about 400 cycles.
-// 16-byte forms: an FP64 instruction takes 64 cycles of a warp's issue on GB300 whatever its active
-// lanes, so the elements of the core are spread over the lanes: lane j carries column k0 + j for
-// the left application, lanes 0 .. 3 the rows k - 1 .. k + 2 for the right one.
+// and the reflector (670 cycles a step with the stores and the next step's loads).
+// Double-float: an operation is 8 to 20 FP32 instructions, so the elements of the core are spread over the
+// lanes: lane j carries column k0 + j for the left application, lanes 0 .. 3 the rows k - 1 .. k + 2 for the
+// right one. (FP64: chase_window64.)
 template <class R>
 __device__ __noinline__ void chase_window(Cx<R>* H, int ldh, const Cx<R>* tile, const Request& rq, QrChase<R>& cs,
                                           QrRecord<R>& g, uint64_t* bars) {

@@ -151,7 +151,8 @@ class BatchInputs:
 
 def solve_batch(conv, inp, precision='double', amplitudes=False, handle=None, out=None):
     """Stages B and C for a batch (wb_solve_batch). Returns ``(R, T, status[, amps])`` with R, T
-    of shape ``(B, 3, n_v, n_u)`` for [given polarization, pure s, pure p]."""
+    of shape ``(B, 3, n_v, n_u)`` for [given polarization, pure s, pure p]. ``precision='double'``
+    computes in FP64, its products normwise accurate to 2^-53 (see WB_PRECISION_FP64 in the C header)."""
     dev = conv.buf.device
     hu, hv = conv.hu, conv.hv
     N = n_orders(hu, hv)
